@@ -170,12 +170,16 @@ int pado_apply_host_terms(const double *f_host, long n1, long n2, long n3, const
 
 /* Launch shape of the line kernels for this handle: m = segment length
  * (rows one thread solves serially, 8/16/32/64), lines = lines per CTA
- * (8/16/32).  0 keeps the current value.  Rebuilds the handle's tables. */
+ * (8/16/32).  0 keeps the current value.  Rebuilds the handle's tables.
+ * After a call that names m or lines the automatic choice keeps to the
+ * kernels that take them; a call with two zeros gives it all of them back. */
 int pado_set_tiling(pado_op_t op, int m, int lines);
 int pado_get_tiling(pado_op_t op, int *m, int *lines);
-/* Kernel organisation of the forward operator: 0 = automatic (the
- * streaming kernel: 4 where the copy engine can move the field, else 6;
- * adjoints of fields 4 cannot take run 1; the default),
+/* Kernel organisation of the forward operator: 0 = automatic (the register
+ * kernel for lines of 24 points or more when no tiling was set, fed by the
+ * copies of 4 where the copy engine can move the field, else by those of 6;
+ * shorter lines and the adjoints of bounded ones: the streaming kernel, 4
+ * or 6; adjoints of fields 4 cannot take run 1; the default),
  * 1 = one CTA per tile of lines, 2 = persistent CTAs that prefetch the next
  * tile with cp.async while the current one is solved, 3 = persistent CTAs
  * that read lines straight into registers and warm L2 with the next tile
@@ -205,7 +209,8 @@ int pado_set_stream_tiling(pado_op_t op, int lines, int stages);
  * memory); clear != 0 resets the word.  No counterpart in the reference. */
 int pado_device_status(pado_op_t op, int clear);
 /* The kernel a forward apply with these arguments would launch (nothing is
- * launched): info[0] kernel variant (1..6), [1] lines per tile, [2] stages,
+ * launched): info[0] kernel variant (1..6; the register kernel: 4 or 6, the
+ * copies that feed it), [1] lines per tile, [2] stages,
  * [3] CTAs per SM, [4] segments per line, [5] coupling window, [6] threads
  * per CTA, [7] dynamic shared memory bytes.  No counterpart in the reference. */
 int pado_launch_plan(pado_op_t op, int kind, int axis, const double *f, double *df, long na, long nb, int bc1,

@@ -17,11 +17,14 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIBDIR = os.path.join(HERE, "_lib")
 LIB = os.path.join(LIBDIR, "libpado.so")
-SOURCES = ["pado_api.cu", "pado_batch.cu", "pado_tables.cpp", "pado_inst.cu", "pado_stagg.cu"]
+SOURCES = ["pado_api.cu", "pado_batch.cu", "pado_tables.cpp", "pado_inst.cu", "pado_stagg.cu",
+           "pado_reg_inst.cu", "pado_reg_tables.cpp"]
 HEADERS = ["pado_common.h", "pado_tables.h", "pado_kernels.cuh", "pado_batch.cuh", "pado_internal.h", "pado_params.h",
-           "pado_stream.cuh", "pado_resident.cuh"]
+           "pado_stream.cuh", "pado_resident.cuh", "pado_reg.cuh", "pado_reg_tables.h"]
 # pado_inst.cu is compiled once per stencil (-DPADO_RK=n) into pado_inst_rkN.o
 STENCILS = 4
+# pado_reg_inst.cu once per stencil and segment length (-DPADO_RM=m) into pado_reg_inst_rkN_m.o
+REG_STENCILS, REG_ROWS = 4, (8, 16, 32)
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2",
               "--expt-relaxed-constexpr"]
@@ -61,6 +64,9 @@ def build(force: bool = False, verbose: bool = False) -> str:
         stem = os.path.splitext(src)[0]
         if src == "pado_inst.cu":
             units += [(src, f"{stem}_rk{rk}.o", [f"-DPADO_RK={rk}"]) for rk in range(STENCILS)]
+        elif src == "pado_reg_inst.cu":
+            units += [(src, f"{stem}_rk{rk}_{m}.o", [f"-DPADO_RK={rk}", f"-DPADO_RM={m}"])
+                      for rk in range(REG_STENCILS) for m in REG_ROWS]
         else:
             units.append((src, stem + ".o", []))
     for src, oname, defs in units:

@@ -66,19 +66,64 @@ void default_tiling(int n, int *m, int *lines)
     *lines = L;
 }
 
-template <typename T>
-int upload_vec(pado_op_s *op, const std::vector<T> &h, T **d)
+// The handle's tables, gathered for one device allocation and one copy (a
+// bounded cd10 object has some 300 of them; one by one their allocations and
+// copies were most of its init).
+struct Upload {
+    std::vector<unsigned char> bytes;
+    std::vector<std::pair<void **, size_t>> at;  // pointer to set, offset
+    template <typename T>
+    void add(const std::vector<T> &h, T **d)
+    {
+        *d = nullptr;
+        if (h.empty()) return;
+        const size_t off = (bytes.size() + 255) / 256 * 256;
+        bytes.resize(off + h.size() * sizeof(T));
+        std::memcpy(bytes.data() + off, h.data(), h.size() * sizeof(T));
+        at.emplace_back(reinterpret_cast<void **>(d), off);
+    }
+    int send(pado_op_s *op)
+    {
+        if (bytes.empty()) return PADO_OK;
+        void *p = nullptr;
+        cudaError_t e = cudaMalloc(&p, bytes.size());
+        if (e != cudaSuccess) return cuda_fail(e);
+        op->allocations.push_back(p);
+        e = cudaMemcpy(p, bytes.data(), bytes.size(), cudaMemcpyHostToDevice);
+        if (e != cudaSuccess) return cuda_fail(e);
+        for (auto &[d, off] : at) *d = static_cast<unsigned char *>(p) + off;
+        return PADO_OK;
+    }
+};
+
+// The register kernel's constants of every operator of the handle.
+void build_reg(pado_op_s *op, const std::vector<int> &kinds, const std::vector<std::pair<int, int>> &bcs, Upload *up)
 {
-    *d = nullptr;
-    if (h.empty()) return PADO_OK;
-    void *p = nullptr;
-    cudaError_t e = cudaMalloc(&p, h.size() * sizeof(T));
-    if (e != cudaSuccess) return cuda_fail(e);
-    op->allocations.push_back(p);
-    e = cudaMemcpy(p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) return cuda_fail(e);
-    *d = static_cast<T *>(p);
-    return PADO_OK;
+    const int n = op->n;
+    if (n < REG_MIN_N) return;
+    auto add = [&](const RegBand &band, int kind, int b1, int bn, int s1, int sn, bool even_starts) {
+        const RegKey key(kind, b1, bn, s1, sn, even_starts ? 1 : 0);
+        if (op->reg.count(key)) return;
+        auto r = std::make_unique<RegOp>();
+        if (!choose_reg_cut(reg_rows(n, op->periodic != 0), even_starts, &r->cut)) return;
+        std::memset(&r->kp, 0, sizeof(r->kp));
+        std::vector<double> tab;
+        const bool own = op->scheme == CD06;  // cd06 takes its closures from init (cd06.F90:177)
+        reg_fill(band, op->scheme, kind, op->dx, op->periodic != 0, own ? op->bc1 : b1, own ? op->bcn : bn,
+                 own ? op->bc1 : s1, own ? op->bcn : sn, r->cut, &r->kp, &tab);
+        r->kp.status = op->d_status;
+        up->add(tab, const_cast<double **>(&r->kp.segtab));
+        op->reg[key] = std::move(r);
+    };
+    for (int kind : kinds) {
+        const RegBand band = RegBand::of(op->scheme, kind, n, op->periodic != 0);
+        for (auto [b1, bn] : bcs)
+            for (bool even : {false, true}) {
+                if (even && n % 2) continue;
+                add(band, kind, b1, bn, b1, bn, even);
+                if (kind == FILTER && !op->periodic && !even) add(band, kind, b1, bn, 0, 0, even);  // complex filter3 (along z)
+            }
+    }
 }
 
 int build_tables(pado_op_s *op)
@@ -86,6 +131,7 @@ int build_tables(pado_op_s *op)
     for (void *p : op->allocations) cudaFree(p);
     op->allocations.clear();
     op->tables.clear();
+    op->reg.clear();
     {
         std::lock_guard<std::mutex> g(op->plan_mu);
         op->plan_cache.clear();  // its keys name the tables
@@ -100,30 +146,30 @@ int build_tables(pado_op_s *op)
     else
         for (int b1 : {0, 1, -1})
             for (int bn : {0, 1, -1}) bcs.push_back({b1, bn});
+    Upload up;
     for (int kind : kinds) {
         for (auto [b1, bn] : bcs) {
             // cd06 takes its closures from init (cd06.F90:177)
             const int cb1 = op->scheme == CD06 ? op->bc1 : b1, cbn = op->scheme == CD06 ? op->bcn : bn;
             for (int dir = 0; dir < 2; ++dir) {
-                DevTables dt;
+                DevTables &dt = op->tables[TabKey(kind, b1, bn, dir)];
                 dt.host = make_op_tables(op->scheme, kind, n, op->dx, op->periodic, cb1, cbn, op->m, dir == 1);
                 const OpTables &h = dt.host;
-                int rc = upload_vec(op, h.tab, &dt.tab);
-                if (rc == PADO_OK) rc = upload_vec(op, h.chain.ctab, &dt.ctab);
-                if (rc == PADO_OK) rc = upload_vec(op, h.chain.xtab, &dt.xtab);
-                if (rc == PADO_OK) rc = upload_vec(op, h.chain_exact.ctab, &dt.ctab_exact);
-                if (rc == PADO_OK) rc = upload_vec(op, h.chain_exact.xtab, &dt.xtab_exact);
-                if (rc == PADO_OK) rc = upload_vec(op, h.etab, &dt.etab);
-                if (rc == PADO_OK) rc = upload_vec(op, h.ktab, &dt.ktab);
-                if (rc == PADO_OK) rc = upload_vec(op, h.rtab, &dt.rtab);
-                if (rc == PADO_OK) rc = upload_vec(op, h.toff, &dt.toff);
-                if (rc == PADO_OK) rc = upload_vec(op, h.bt, &dt.bt);
-                if (rc != PADO_OK) return rc;
-                op->tables[TabKey(kind, b1, bn, dir)] = std::move(dt);
+                up.add(h.tab, &dt.tab);
+                up.add(h.chain.ctab, &dt.ctab);
+                up.add(h.chain.xtab, &dt.xtab);
+                up.add(h.chain_exact.ctab, &dt.ctab_exact);
+                up.add(h.chain_exact.xtab, &dt.xtab_exact);
+                up.add(h.etab, &dt.etab);
+                up.add(h.ktab, &dt.ktab);
+                up.add(h.rtab, &dt.rtab);
+                up.add(h.toff, &dt.toff);
+                up.add(h.bt, &dt.bt);
             }
         }
     }
-    return PADO_OK;
+    build_reg(op, kinds, bcs, &up);
+    return up.send(op);
 }
 
 KernelFn pick_kernel(int rk, bool per, bool adj, bool contiguous, int m, int variant)
@@ -185,14 +231,14 @@ int stream_tile_doubles(bool xl, int n, int L, bool as)
 }
 
 // Lets a streaming kernel use up to 227 KB of shared memory (once per kernel).
-bool grant_smem(StreamFn fn)
+bool grant_smem(const void *fn)
 {
     static std::mutex mu;
     static std::map<const void *, bool> granted;
     std::lock_guard<std::mutex> g(mu);
-    bool &ok = granted[(const void *)fn];
+    bool &ok = granted[fn];
     if (!ok) {
-        if (cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) !=
+        if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) !=
             cudaSuccess) {
             (void)cudaGetLastError();
             return false;
@@ -235,7 +281,7 @@ bool choose_stream_tiling(const pado_op_s *op, const DevTables &dt, const KParam
         if (op->stream_lines && L != op->stream_lines) continue;
         if (op->stream_stages && stages != op->stream_stages) continue;
         StreamFn fn = pick_stream(kp0.rc.rk, op->periodic != 0, op->m, xl, L, adj, as);
-        if (!grant_smem(fn)) continue;
+        if (!grant_smem((const void *)fn)) continue;
         const int tile_doubles = stream_tile_doubles(xl, n, L, as);
         const size_t bytes = stream_smem_bytes(L, S, kp0.xd, stages, tile_doubles, etab_rows, ktab_rows, resp_rows(kp0));
         if (bytes > 227 * 1024) continue;
@@ -317,7 +363,7 @@ bool plan_stream(const pado_op_s *op, const DevTables &dt, const KParams &kp0, i
     const int best_slots = choice.nslots, best_ctas = choice.ctas;
     unsigned char best_perm[KMAXSLOT];
     std::memcpy(best_perm, choice.perm, sizeof(best_perm));
-    if (!grant_smem(pick_stream(kp0.rc.rk, op->periodic != 0, op->m, xl, choice.L, adj, as))) return false;
+    if (!grant_smem((const void *)pick_stream(kp0.rc.rk, op->periodic != 0, op->m, xl, choice.L, adj, as))) return false;
     const int L = choice.L, stages = choice.stages;
     const int tile_doubles = stream_tile_doubles(xl, n, L, as);
     std::memset(sp, 0, sizeof(*sp));
@@ -372,6 +418,39 @@ bool plan_stream(const pado_op_s *op, const DevTables &dt, const KParams &kp0, i
     return true;
 }
 
+bool plan_reg_op(const pado_op_s *op, const RegOp &ro, const KParams &kp0, int axis, long long na, long long nb, bool adj,
+                 RegLaunch *out)
+{
+    RegParams &kp = out->kp;
+    kp = ro.kp;
+    kp.in = kp0.in;
+    kp.out = kp0.out;
+    kp.nlines = kp0.nlines;
+    kp.stride = kp0.stride;
+    kp.axis = axis;
+    kp.out_mode = kp0.out_mode;
+    kp.out_alpha = kp0.out_alpha;
+    const int rk = kp0.rc.rk;
+    if (adj && (rk == RHS_CD06_D1 || rk == RHS_CD10_D1))
+        for (double &t : kp.taps) t = -t;  // a cyclic first derivative is antisymmetric, the others symmetric
+    return plan_reg(rk, op->periodic != 0, ro.cut, na, nb, out);
+}
+
+// The register kernel's constants for a request, or null when another kernel
+// runs it: an explicit kernel or tiling, a short or uncuttable line, the
+// adjoint of a bounded line.
+const RegOp *reg_op(const pado_op_s *op, int kind, int axis, const double *f, const double *df, int bc1, int bcn,
+                    bool adj, int solve_bc1, int solve_bcn)
+{
+    if (op->variant != 0 || op->stream_lines || op->stream_stages || op->tiled || (adj && !op->periodic)) return nullptr;
+    const bool bounded_bc = !op->periodic && op->scheme != CD06;
+    const int b1 = bounded_bc ? bc1 : 0, bn = bounded_bc ? bcn : 0;
+    const int s1 = bounded_bc && solve_bc1 != SAME_BC ? solve_bc1 : b1, sn = bounded_bc && solve_bcn != SAME_BC ? solve_bcn : bn;
+    const bool even = axis == 1 && op->n % 2 == 0 && !((reinterpret_cast<size_t>(f) | reinterpret_cast<size_t>(df)) & 15);
+    const auto it = op->reg.find(RegKey(kind, b1, bn, s1, sn, even ? 1 : 0));
+    return it == op->reg.end() ? nullptr : it->second.get();
+}
+
 int sm_count()
 {
     int dev = 0, sms = 0;
@@ -393,6 +472,159 @@ int launch_stream(pado_op_s *op, const StreamParams &sp, bool adj, int threads, 
 }
 
 }  // namespace
+
+namespace pado {
+
+// Rows per segment of the register kernel for a line of `rows` rows to cover:
+// the longest segments the line cuts into.  Each halves the halo reads, the
+// link / close steps and the barriers per row of the next shorter one: 512
+// rows run 5-20% faster with 32 than with 16 (B200, all stencils and axes),
+// 64 to 128 rows within 5% of each other, 8 rows 10-50% slower.
+bool choose_reg_cut(int rows, bool even_starts, RegCut *cut)
+{
+    for (int M : {32, 16, 8})
+        if (reg_cut(rows, M, even_starts, cut)) return true;
+    return false;
+}
+
+RegFn pick_reg(int rk, int m, bool per, bool even, int mode, int lines)
+{
+#define PADO_REG_M(rk)                                                     \
+    (m == 8 ? pick_reg_rk##rk##_8(per, even, mode, lines)                  \
+            : (m == 16 ? pick_reg_rk##rk##_16(per, even, mode, lines) : pick_reg_rk##rk##_32(per, even, mode, lines)))
+    switch (rk) {
+    case RHS_CD06_D1: return PADO_REG_M(0);
+    case RHS_CD10_D1: return PADO_REG_M(1);
+    case RHS_CD10_D2: return PADO_REG_M(2);
+    default: return PADO_REG_M(3);
+    }
+#undef PADO_REG_M
+}
+
+// CTAs per SM of a kernel with the given launch shape (0: it does not run),
+// asked of the runtime once per shape and device.
+int resident_ctas(const void *fn, int threads, size_t smem)
+{
+    static std::mutex mu;
+    static std::map<std::tuple<const void *, int, size_t, int>, int> known;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const std::tuple<const void *, int, size_t, int> key(fn, threads, smem, dev);
+    std::lock_guard<std::mutex> g(mu);
+    const auto it = known.find(key);
+    if (it != known.end()) return it->second;
+    int ctas = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, fn, threads, smem) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return 0;
+    }
+    return known[key] = ctas;
+}
+
+bool plan_reg(int rk, bool per, const RegCut &cut, long long na, long long nb, RegLaunch *out)
+{
+    RegParams &kp = out->kp;
+    const int n = kp.n, nin = kp.nin, S = cut.S, M = cut.M, axis = kp.axis;
+    if (na > 0x7fffffffLL || nb > 0x7fffffffLL || kp.nlines > 0x7fffffffLL) return false;
+    const size_t align_bits = reinterpret_cast<size_t>(kp.in) | reinterpret_cast<size_t>(kp.out);
+    if (align_bits & 7) return false;
+    const bool xl = axis == 1;
+    const bool tma_ok = !(align_bits & 15) && (xl ? n % 2 == 0 : na % 2 == 0);
+    const int mode = xl ? (tma_ok ? REG_SWZ : REG_PACK) : REG_ROWS;
+    const bool even = per && cut.even();
+    // Lines per tile, measured on 2^25..2^26 points (GB/s).  Strided lines: as
+    // many as 512 threads sweep (longer rows for the copy engine and DRAM:
+    // cd10 d1 along z, n = 512, 32 lines 5440, 16 lines 5160; n = 1024, 16
+    // lines 5340, 8 lines 4520), but 256 threads for cf90 above 16 lines, whose
+    // longer link and close steps need a second CTA to hide (n = 512 bounded:
+    // 16 lines 4790, 32 lines 4140).  x lines: 8, with a second buffer the
+    // copies fill meanwhile (cd10 d1, n = 512 bounded: 5640 against 5030 with
+    // 16 lines); 16 for short lines, which give 8 lines too few threads (n =
+    // 64 bounded: 4490 against 3490).
+    int L = S * 32 <= 512 ? 32 : (S * 16 <= 512 ? 16 : 8);
+    if (rk == RHS_CF90 && L * S > 256 && L > 16) L = 16;
+    if (mode != REG_ROWS && L > 16) L = 16;
+    if (mode == REG_SWZ && n > 128) L = 8;
+    int stages = mode == REG_SWZ ? 2 : 1;
+    const int max_threads = M >= 32 ? 512 : 384;
+    while (L > 8 && L * S > max_threads) L /= 2;
+    const int threads = (L * S + 31) / 32 * 32;
+    if (threads > max_threads) return false;
+    kp.stages = stages;
+    kp.P = n | 1;
+    if (xl) {
+        kp.ntiles = (kp.nlines + L - 1) / L;
+        kp.chunks = n / 16;
+        kp.tile_doubles = mode == REG_SWZ ? (n + 15) / 16 * 16 * L : round16((long long)kp.P * L);
+    } else {
+        kp.na = (int)na;
+        kp.xblocks = (int)((na + L - 1) / L);
+        kp.ntiles = (long long)kp.xblocks * nb;
+        kp.pstride = axis == 2 ? na * (long long)nin : na;
+        kp.async_copy = tma_ok ? 0 : 1;
+        kp.nbox = (nin + 255) / 256;
+        kp.box_rows = ((nin + kp.nbox - 1) / kp.nbox + 15) / 16 * 16;
+        kp.tile_doubles = (tma_ok ? kp.nbox * kp.box_rows : (nin + 15) / 16 * 16) * L;
+    }
+    if (kp.ntiles > 0x7fffffffLL) return false;
+    const int edge_table = reg_edge_table(rk, per, S);
+    out->smem = reg_smem_bytes(L, S, stages, kp.tile_doubles, edge_table);
+    while (stages > 1 && out->smem > 227 * 1024) {
+        kp.stages = stages = 1;
+        out->smem = reg_smem_bytes(L, S, stages, kp.tile_doubles, edge_table);
+    }
+    if (out->smem > 227 * 1024) return false;
+    out->fn = pick_reg(rk, M, per, even, mode, L);
+    if (!grant_smem((const void *)out->fn)) return false;
+    const int ctas = resident_ctas((const void *)out->fn, threads, out->smem);
+    if (ctas < 1) return false;
+    if (tma_ok) {
+        EncodeTiledFn enc = encode_tiled();
+        if (!enc) return false;
+        auto map = [&](CUtensorMap *m, const double *p, int rank, const cuuint64_t *dims, const cuuint64_t *strides,
+                       const cuuint32_t *box, CUtensorMapSwizzle swz) {
+            const cuuint32_t ones[3] = {1, 1, 1};
+            return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, (cuuint32_t)rank, const_cast<double *>(p), dims, strides, box,
+                       ones, CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+        };
+        if (xl) {
+            const cuuint64_t d3[3] = {16, (cuuint64_t)kp.nlines, (cuuint64_t)kp.chunks}, s3[2] = {(cuuint64_t)n * 8, 128};
+            const cuuint32_t b3[3] = {16, (cuuint32_t)L, (cuuint32_t)kp.chunks};
+            if (kp.chunks && !(map(&kp.tin, kp.in, 3, d3, s3, b3, CU_TENSOR_MAP_SWIZZLE_128B) &&
+                               map(&kp.tout, kp.out, 3, d3, s3, b3, CU_TENSOR_MAP_SWIZZLE_128B)))
+                return false;
+            const cuuint64_t d2[2] = {(cuuint64_t)n, (cuuint64_t)kp.nlines}, s2[1] = {(cuuint64_t)n * 8};
+            const cuuint32_t b2[2] = {16, (cuuint32_t)L};
+            if (n % 16 && !(map(&kp.tin2, kp.in, 2, d2, s2, b2, CU_TENSOR_MAP_SWIZZLE_128B) &&
+                            map(&kp.tout2, kp.out, 2, d2, s2, b2, CU_TENSOR_MAP_SWIZZLE_128B)))
+                return false;
+        } else {
+            const cuuint64_t dims[3] = {(cuuint64_t)na, (cuuint64_t)(axis == 2 ? nin : nb), (cuuint64_t)(axis == 2 ? nb : nin)};
+            const cuuint64_t strides[2] = {(cuuint64_t)na * 8, (cuuint64_t)na * (axis == 2 ? nin : nb) * 8};
+            const cuuint32_t box[3] = {(cuuint32_t)L, (cuuint32_t)(axis == 2 ? kp.box_rows : 1),
+                                       (cuuint32_t)(axis == 2 ? 1 : kp.box_rows)};
+            if (!map(&kp.tin, kp.in, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE)) return false;
+        }
+    }
+    out->threads = threads;
+    out->ctas = ctas;
+    out->lines = L;
+    out->mode = mode;
+    return true;
+}
+
+int launch_reg(const RegLaunch &r, cudaStream_t st)
+{
+    const long long grid = std::min<long long>(r.kp.ntiles, (long long)r.ctas * sm_count());
+    if (grid < 1) return PADO_OK;
+    r.fn<<<(unsigned)grid, r.threads, r.smem, st>>>(r.kp);
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? PADO_OK : cuda_fail(e);
+}
+
+}  // namespace pado
 
 int pado::prepare_launch(pado_op_s *op, int kind, int axis, const double *f, double *df, long na, long nb, int bc1,
                          int bcn, bool adjoint, int lines, bool no_fast, KParams *kpo, bool *trivial, int solve_bc1,
@@ -481,6 +713,10 @@ int launch(pado_op_s *op, int kind, int axis, const double *f, double *df, long 
             e = cudaGetLastError();
         }
         return e == cudaSuccess ? PADO_OK : cuda_fail(e);
+    }
+    if (const RegOp *ro = reg_op(op, kind, axis, f, df, bc1, bcn, adjoint, solve_bc1, solve_bcn)) {
+        RegLaunch r;
+        if (plan_reg_op(op, *ro, kp, axis, na, nb, adjoint, &r)) return launch_reg(r, st);
     }
     if (op->variant == 0 || op->variant == 4 || op->variant == 6) {
         const bool bounded_bc = !op->periodic && op->scheme != CD06;
@@ -843,6 +1079,7 @@ int pado_set_tiling(pado_op_t op, int m, int lines)
     const int om = op->m, ol = op->lines;
     if (m) op->m = m;
     if (lines) op->lines = lines;
+    op->tiled = m != 0 || lines != 0;
     const int S = (op->n + op->m - 1) / op->m;
     if (S > 32) {
         op->m = om;
@@ -870,6 +1107,21 @@ int pado_launch_plan(pado_op_t op, int kind, int axis, const double *f, double *
     bool trivial = true;
     int rc = prepare_launch(op, kind, axis, f, df, na, nb, bc1, bcn, false, op ? op->lines : 0, false, &kp, &trivial);
     if (rc != PADO_OK || trivial) return rc;
+    if (const RegOp *ro = reg_op(op, kind, axis, f, df, bc1, bcn, false, SAME_BC, SAME_BC)) {
+        RegLaunch r;
+        if (plan_reg_op(op, *ro, kp, axis, na, nb, false, &r)) {
+            const bool copies = axis == 1 ? r.mode == REG_PACK : r.kp.async_copy != 0;
+            info[0] = copies ? 6 : 4;
+            info[1] = r.lines;
+            info[2] = r.kp.stages;
+            info[3] = r.ctas;
+            info[4] = r.kp.S;
+            info[5] = r.kp.W;
+            info[6] = r.threads;
+            info[7] = (int)r.smem;
+            return PADO_OK;
+        }
+    }
     info[4] = kp.S;
     info[5] = kp.W;
     if (op->variant == 0 || op->variant == 4 || op->variant == 6) {

@@ -26,7 +26,13 @@ enum Scheme { CD06 = 0, CD10 = 1, CF90 = 2 };
 enum Kind { FILTER = 0, D1 = 1, D2 = 2 };
 
 // Which explicit stencil a kernel applies.
-enum RhsKind { RHS_CD06_D1 = 0, RHS_CD10_D1 = 1, RHS_CD10_D2 = 2, RHS_CF90 = 3 };
+// RHS_ST_*: the staggered scheme's -- from edges to the cells between them
+// and back (two differences, or two sums, of values at half cells), and the
+// collocated first and second derivatives.
+enum RhsKind {
+    RHS_CD06_D1 = 0, RHS_CD10_D1 = 1, RHS_CD10_D2 = 2, RHS_CF90 = 3,
+    RHS_ST_EC = 4, RHS_ST_CE = 5, RHS_ST_D1 = 6, RHS_ST_D2 = 7
+};
 
 PADO_HD PADO_INLINE int rhs_kind_of(int scheme, int kind)
 {
@@ -205,6 +211,16 @@ PADO_HD PADO_INLINE double rhs_interior_fma(int rk, int periodic, const double *
     case RHS_CD10_D2: {
         const double m2 = -2.0 * v[4];
         return fma(c[2], v[7] + m2 + v[1], fma(c[1], v[6] + m2 + v[2], c[0] * (v[5] + m2 + v[3])));
+    }
+    case RHS_ST_EC:
+    case RHS_ST_CE:
+        // v[4], v[5]: the two nearest points; c[2]: -1 (derivative) or 1 (interpolation)
+        return fma(c[0], fma(c[2], v[4], v[5]), c[1] * fma(c[2], v[3], v[6]));
+    case RHS_ST_D1:
+        return fma(c[0], v[5] - v[3], c[1] * (v[6] - v[2]));
+    case RHS_ST_D2: {
+        const double m2 = -2.0 * v[4];
+        return fma(c[1], v[6] + m2 + v[2], c[0] * (v[5] + m2 + v[3]));
     }
     default:
         return fma(c[4], v[8] + v[0],

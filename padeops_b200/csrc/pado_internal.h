@@ -5,6 +5,7 @@
 
 #include <atomic>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <tuple>
 #include <vector>
@@ -12,6 +13,7 @@
 #include "../../include/pado.h"
 #include "pado_kernels.cuh"
 #include "pado_params.h"
+#include "pado_reg_tables.h"
 #include "pado_stream.cuh"
 #include "pado_tables.h"
 
@@ -35,6 +37,14 @@ struct DevTables {
     double *bt = nullptr;          // transposed stencil blocks (adjoint, bounded)
 };
 
+// The register kernel's constants for one (kind, closures) operator: launch
+// parameters with every table filled in, geometry and pointers left to the
+// launch.
+struct RegOp {
+    RegCut cut;
+    RegParams kp;
+};
+
 using TabKey = std::tuple<int, int, int, int>;  // kind, bc1, bcn, adjoint
 
 // The streaming kernel's tiling for one (tables, line direction, copy path,
@@ -45,6 +55,8 @@ struct StreamChoice {
     int L = 0, stages = 0, ctas = 0, nslots = 0;
     unsigned char perm[KMAXSLOT] = {0};
 };
+// kind, closures of the right-hand side, closures of the system solved, even segment starts
+using RegKey = std::tuple<int, int, int, int, int, int>;
 using PlanKey = std::tuple<const void *, int, int, int, int, int>;  // tables, x lines, async, adjoint, lines, stages
 
 int cuda_fail(cudaError_t e);
@@ -57,6 +69,7 @@ struct pado_op_s {
     int scheme = 0, n = 0, periodic = 1, bc1 = 0, bcn = 0;
     double dx = 1.0;
     int m = 32, lines = 16;
+    bool tiled = false;  // the caller asked for a tiling (pado_set_tiling)
     int variant = 0;  // 0: automatic; 1..3: one-CTA-per-tile / persistent kernels; 4: streaming kernel
     int device = 0;
     int *d_status = nullptr;  // device-side status word (bounded waits)
@@ -64,6 +77,7 @@ struct pado_op_s {
     mutable std::mutex plan_mu;                                      // guards plan_cache
     mutable std::map<pado::PlanKey, pado::StreamChoice> plan_cache;  // the planner's choices
     std::map<pado::TabKey, pado::DevTables> tables;
+    std::map<pado::RegKey, std::unique_ptr<pado::RegOp>> reg;  // register kernel; empty when the line does not cut
     std::vector<void *> allocations;
     // host-buffer staging
     std::mutex staging_mu;
@@ -92,6 +106,34 @@ StreamFn pick_stream_rk0(bool per, int m, bool xl, int lines, bool adj, bool as)
 StreamFn pick_stream_rk1(bool per, int m, bool xl, int lines, bool adj, bool as);
 StreamFn pick_stream_rk2(bool per, int m, bool xl, int lines, bool adj, bool as);
 StreamFn pick_stream_rk3(bool per, int m, bool xl, int lines, bool adj, bool as);
+
+// register kernel (pado_reg_inst.cu): even: the segments share no rows (cyclic lines); mode: RegMode
+using RegFn = void (*)(const RegParams);
+#define PADO_REG_PICK(rk)                                                  \
+    RegFn pick_reg_rk##rk##_8(bool per, bool even, int mode, int lines);  \
+    RegFn pick_reg_rk##rk##_16(bool per, bool even, int mode, int lines); \
+    RegFn pick_reg_rk##rk##_32(bool per, bool even, int mode, int lines);
+PADO_REG_PICK(0)
+PADO_REG_PICK(1)
+PADO_REG_PICK(2)
+PADO_REG_PICK(3)
+#undef PADO_REG_PICK
+RegFn pick_reg(int rk, int m, bool per, bool even, int mode, int lines);
+
+// Launch of the register kernel.
+struct RegLaunch {
+    RegParams kp;
+    RegFn fn = nullptr;
+    int threads = 0, ctas = 0, lines = 0, mode = 0;
+    size_t smem = 0;
+};
+// The cut of a line of `rows` rows to cover into the longest segments it takes.
+bool choose_reg_cut(int rows, bool even_starts, RegCut *cut);
+// Plans the lines along `axis` of a field of the given geometry (out->kp: in,
+// out, nlines, stride, axis and output mode set on top of the operator's
+// constants); false when the field or line does not fit.
+bool plan_reg(int rk, bool per, const RegCut &cut, long long na, long long nb, RegLaunch *out);
+int launch_reg(const RegLaunch &r, cudaStream_t st);
 
 // no_fast: every segment on the per-row table (for kernels built for a
 // segment length other than the handle's).

@@ -99,7 +99,8 @@ class _Scheme:
         check(L.lib().pado_set_tiling(self.handle, m, lines), "set_tiling")
 
     def set_variant(self, variant: int) -> None:
-        """0 = automatic, 1 = one CTA per tile of lines, 2/3 = persistent CTAs
+        """0 = automatic (the register kernel where the line cuts into its
+        segments and no tiling was set), 1 = one CTA per tile of lines, 2/3 = persistent CTAs
         with prefetch, 4 = the streaming (TMA-fed) kernel, 5 = its resident
         tiles fed by plain loads, 6 = the streaming kernel fed by per-element
         asynchronous copies (5 and 6: any extent and 8-byte alignment)."""

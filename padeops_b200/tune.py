@@ -22,7 +22,8 @@ from . import _lib as L
 _CACHE_LOCK = threading.Lock()
 M_CHOICES = (16, 32, 64)
 LINE_CHOICES = (8, 16, 32)
-VARIANTS = (4, 6, 5, 1, 2, 3)  # 4, 6, 5: streaming kernel's resident tiles (they pick their own lines per tile)
+# 0: the automatic choice (no tiling); 4, 6, 5: streaming kernel's resident tiles (they pick their own lines per tile)
+VARIANTS = (0, 4, 6, 5, 1, 2, 3)
 
 
 def cache_path() -> str:
@@ -52,7 +53,7 @@ def _store(d: dict) -> None:
 
 def _key(op, kind: int, axis: int, shape: tuple[int, int, int]) -> str:
     gpu = torch.cuda.get_device_name()
-    return f"{gpu}|scheme={op._scheme}|kind={kind}|n={op.n}|per={int(op.periodic)}|axis={axis}|shape={shape}"
+    return f"{gpu}|v2|scheme={op._scheme}|kind={kind}|n={op.n}|per={int(op.periodic)}|axis={axis}|shape={shape}"
 
 
 def time_op(op, kind: int, axis: int, f: torch.Tensor, df: torch.Tensor, na: int, nb: int, reps: int = 5,
@@ -72,7 +73,7 @@ def tune_op(op, kind: int, axis: int, shape: tuple[int, int, int], reps: int = 5
             verbose: bool = False) -> tuple[int, int, float]:
     """Pick the fastest (m, lines, kernel variant) for `op` applied along `axis`
     of a field of shape (n3, n2, n1) and set it on the handle.
-    Returns (m, lines, variant, ms)."""
+    Returns (m, lines, variant, ms); (0, 0, 0, ms) is the automatic choice."""
     key = _key(op, kind, axis, tuple(shape))
     if use_cache:
         with _CACHE_LOCK:
@@ -87,10 +88,11 @@ def tune_op(op, kind: int, axis: int, shape: tuple[int, int, int], reps: int = 5
     f = torch.randn(n3 * n2 * n1, dtype=torch.float64, device="cuda", generator=g)
     df = torch.empty_like(f)
     best = None
+    m0, lines0 = op.get_tiling()
     for variant in VARIANTS:
         op.set_variant(variant)
-        for m in M_CHOICES:
-            for lines in ((0,) if variant in (4, 5, 6) else LINE_CHOICES):
+        for m in M_CHOICES if variant else (0,):
+            for lines in ((0,) if variant in (0, 4, 5, 6) else LINE_CHOICES):
                 try:
                     op.set_tiling(m, lines)
                     ms = time_op(op, kind, axis, f, df, na, nb, reps)
@@ -104,6 +106,8 @@ def tune_op(op, kind: int, axis: int, shape: tuple[int, int, int], reps: int = 5
     if best is None:
         raise L.PadoError(L.E_SIZE, "no legal tiling")
     op.set_variant(best[2])
+    if best[2] == 0:
+        op.set_tiling(m0, lines0)  # the handle's own, then no explicit tiling
     op.set_tiling(best[0], best[1])
     if use_cache:
         with _CACHE_LOCK:

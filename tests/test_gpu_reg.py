@@ -1,0 +1,70 @@
+"""GPU: the register kernel (the automatic choice for lines of 24 points and
+more) on fields of more tiles than resident CTAs, at line lengths on the edges
+of its cuts -- no shared rows, the most, one segment -- and partial tiles and
+chunks, through both copy paths, against the oracle (1e-12 of max |oracle|);
+and the same field through the streaming kernel, the path it replaced."""
+import numpy as np
+import pytest
+
+import oracle
+from tests.fields import na_nb, rel_err
+from tests.test_gpu_parity import OPS, _make, _oracle_apply
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-12
+
+
+def _shape(n, axis, odd):
+    e = 1 if odd else 0
+    return {1: (61, 83, n), 2: (37, n, 70 + e), 3: (n, 37, 70 + e)}[axis]
+
+
+@pytest.mark.parametrize("scheme,kind", OPS)
+@pytest.mark.parametrize("n", [24, 31, 32, 50, 64, 72, 127, 128, 200])
+def test_register_kernel(scheme, kind, n):
+    import torch
+
+    rng = np.random.default_rng(11 + n + 3 * scheme + kind)
+    for periodic in (True, False):
+        op = _make(scheme, n, 0.3, periodic)
+        bc = (0, 0) if periodic or scheme == oracle.CD06 else [(0, 0), (1, -1), (-1, 1)][n % 3]
+        for axis in (1, 2, 3):
+            for odd in (False, True) if axis != 1 else (n % 2 == 1,):
+                shape = _shape(n, axis, odd)
+                f = rng.standard_normal(shape)
+                ft = torch.from_numpy(f).cuda()
+                na, nb = na_nb(shape, axis)
+                out = torch.full_like(ft, float("nan"))
+                plan = op.launch_plan(kind, axis, ft, out, na, nb, *bc)
+                assert plan["variant"] == (6 if odd else 4)
+                op.apply(kind, axis, ft, out, na, nb, *bc)
+                torch.cuda.synchronize()
+                assert op.device_status() == 0
+                ref = _oracle_apply(scheme, kind, axis, f, 0.3, periodic, *bc)
+                assert rel_err(out.cpu().numpy(), ref) <= TOL, (periodic, axis, odd)
+                general = torch.full_like(ft, float("nan"))
+                op.set_variant(plan["variant"])
+                op.apply(kind, axis, ft, general, na, nb, *bc)
+                op.set_variant(0)
+                assert rel_err(out.cpu().numpy(), general.cpu().numpy()) <= TOL, (periodic, axis, odd)
+
+
+@pytest.mark.parametrize("scheme,kind", OPS)
+@pytest.mark.parametrize("n", [1000, 1024, 2048])
+def test_register_kernel_long_lines(scheme, kind, n):
+    import torch
+
+    rng = np.random.default_rng(n + 3 * scheme + kind)
+    for periodic in (True, False):
+        op = _make(scheme, n, 0.3, periodic)
+        for axis, shape in ((1, (3, 7, n)), (2, (2, n, 18)), (3, (n, 3, 18))):
+            f = rng.standard_normal(shape)
+            ft = torch.from_numpy(f).cuda()
+            na, nb = na_nb(shape, axis)
+            out = torch.full_like(ft, float("nan"))
+            op.apply(kind, axis, ft, out, na, nb)
+            torch.cuda.synchronize()
+            assert op.device_status() == 0
+            ref = _oracle_apply(scheme, kind, axis, f, 0.3, periodic, 0, 0)
+            assert rel_err(out.cpu().numpy(), ref) <= TOL, (periodic, axis)

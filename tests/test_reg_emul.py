@@ -1,0 +1,94 @@
+"""CPU emulation of the register kernel: its phase functions
+(padeops_b200/csrc/pado_reg.cuh) compiled for the host and run phase by phase
+over every thread (tests/emul/pado_reg_emul.cu), against the oracle -- every
+segment length and tile layout, line lengths at the edges of the cuts (one
+segment, none, the most shared rows), closures, output modes.  Bar: 1e-12 of
+max |oracle|, as everywhere."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import oracle
+
+OPS = [(oracle.CD06, oracle.D1), (oracle.CD10, oracle.D1), (oracle.CD10, oracle.D2), (oracle.CF90, oracle.FILTER)]
+ROWS, SWZ, PACK = 0, 1, 2
+
+
+@pytest.fixture(scope="module")
+def emul():
+    from tests.emul.build_reg import build
+
+    lib = ctypes.CDLL(build())
+    P, I, D, Lg = ctypes.c_void_p, ctypes.c_int, ctypes.c_double, ctypes.c_long
+    lib.emul_reg.argtypes = [I, I, I, D, I, I, I, I, I, I, I, I, I, D, P, P, Lg, Lg]
+    lib.emul_reg_stagg.argtypes = [I, I, I, I, I, P, P, P, I, P, P, Lg]
+    return lib
+
+
+def _run(emul, scheme, kind, n, dx, periodic, bc, solve, m, mode, axis, out_mode, alpha, f, out):
+    na, nb = [s for a, s in enumerate(f.shape[::-1]) if a != axis - 1]
+    return emul.emul_reg(scheme, kind, n, dx, int(periodic), *bc, *solve, m, mode, axis, out_mode, alpha, f.ctypes.data,
+                out.ctypes.data, na, nb)
+
+
+@pytest.mark.parametrize("scheme,kind", OPS)
+@pytest.mark.parametrize("periodic", [True, False])
+def test_register_kernel_emulated(emul, scheme, kind, periodic):
+    rng = np.random.default_rng(31 + scheme + 5 * kind)
+    dx = 0.37
+    cuts = 0
+    # 24: the shortest; 32, 64, 128: no shared rows; 40, 36: the most; 100, 129, 255, 512: both overlaps
+    for n in (24, 25, 32, 36, 40, 64, 100, 129, 255, 512):
+        bcs = [(0, 0)] if periodic or scheme == oracle.CD06 else [(0, 0), (1, -1), (-1, 1)]
+        for bc in bcs:
+            op = oracle.OracleOp(scheme, n, dx, periodic, *bc)
+            for axis, mode in ((1, SWZ), (1, PACK), (2, ROWS), (3, ROWS)):
+                f = rng.standard_normal({1: (3, 5, n), 2: (2, n, 11), 3: (n, 2, 11)}[axis])
+                na, nb = [s for a, s in enumerate(f.shape[::-1]) if a != axis - 1]
+                ref = op.apply(kind, axis, f, na, nb, *bc).reshape(f.shape)
+                for m in (8, 16, 32):
+                    if mode == SWZ and n % 2:
+                        continue
+                    out = np.full_like(f, np.nan)
+                    rc = _run(emul, scheme, kind, n, dx, periodic, bc, bc, m, mode, axis, 0, 1.0, f, out)
+                    if rc == -2:
+                        continue  # the line does not cut into segments of m rows
+                    assert rc == 0
+                    cuts += 1
+                    err = np.abs(out - ref).max() / np.abs(ref).max()
+                    assert err <= 1e-12, (n, m, mode, axis, bc, err)
+    assert cuts > 60
+
+
+def test_register_kernel_output_modes_emulated(emul):
+    rng = np.random.default_rng(5)
+    n = 72
+    for scheme, kind in OPS:
+        op = oracle.OracleOp(scheme, n, 0.2, False)
+        for axis, mode in ((1, SWZ), (1, PACK), (3, ROWS)):
+            f = rng.standard_normal({1: (3, 5, n), 3: (n, 2, 11)}[axis])
+            na, nb = [s for a, s in enumerate(f.shape[::-1]) if a != axis - 1]
+            ref = op.apply(kind, axis, f, na, nb).reshape(f.shape)
+            df0 = rng.standard_normal(f.shape)
+            for out_mode, beta in ((1, 0.0), (2, 1.0)):
+                out = df0.copy()
+                assert _run(emul, scheme, kind, n, 0.2, False, (0, 0), (0, 0), 16, mode, axis, out_mode, -0.75, f, out) == 0
+                expect = -0.75 * ref + beta * df0
+                assert np.abs(out - expect).max() / np.abs(expect).max() <= 1e-12, (scheme, kind, mode, out_mode)
+
+
+def test_register_kernel_other_system_emulated(emul):
+    """The complex z filter: closures in the right-hand side, the (0, 0) system solved."""
+    from oracle import dense
+
+    rng = np.random.default_rng(6)
+    n = 60
+    A = dense.lhs(dense.CF90, dense.FILTER, n, False, 0, 0)
+    for bc in ((1, -1), (-1, 1), (0, 1)):
+        D = np.linalg.solve(A, dense.rhs(dense.CF90, dense.FILTER, n, 1.0, False, *bc))
+        f = rng.standard_normal((n, 2, 11))
+        out = np.empty_like(f)
+        assert _run(emul, dense.CF90, dense.FILTER, n, 1.0, False, bc, (0, 0), 16, ROWS, 3, 0, 1.0, f, out) == 0
+        ref = dense.apply_axis(D, f, 3)
+        assert np.abs(out - ref).max() / np.abs(ref).max() <= 1e-12, bc
