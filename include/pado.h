@@ -325,6 +325,10 @@ int pado_cd06stagg_init_nonperiodic(pado_stagg_t *stagg, int nx, double dx, int 
  * object (the reference solves them with tables its periodic init never
  * allocates). */
 int pado_cd06stagg_sizes(pado_stagg_t stagg, int op, int *nin, int *nout);
+/* Device-side status of the object's kernels: PADO_OK, or PADO_E_TIMEOUT when
+ * a bounded wait for tile copies expired (the output is then incomplete).
+ * Synchronous.  No counterpart in the reference. */
+int pado_cd06stagg_status(pado_stagg_t stagg);
 /* df(n1, n2, nout) = op applied along z to f(n1, n2, nin): device pointers,
  * enqueued on `stream`; f and df must not overlap.  A complex field is
  * passed as its (re, im) doubles with n1 doubled (the coefficients are

@@ -24,7 +24,7 @@ HEADERS = ["pado_common.h", "pado_tables.h", "pado_kernels.cuh", "pado_batch.cuh
 # pado_inst.cu is compiled once per stencil (-DPADO_RK=n) into pado_inst_rkN.o
 STENCILS = 4
 # pado_reg_inst.cu once per stencil and segment length (-DPADO_RM=m) into pado_reg_inst_rkN_m.o
-REG_STENCILS, REG_ROWS = 4, (8, 16, 32)
+REG_STENCILS, REG_ROWS = 8, (8, 16, 32)
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2",
               "--expt-relaxed-constexpr"]

@@ -496,7 +496,11 @@ RegFn pick_reg(int rk, int m, bool per, bool even, int mode, int lines)
     case RHS_CD06_D1: return PADO_REG_M(0);
     case RHS_CD10_D1: return PADO_REG_M(1);
     case RHS_CD10_D2: return PADO_REG_M(2);
-    default: return PADO_REG_M(3);
+    case RHS_CF90: return PADO_REG_M(3);
+    case RHS_ST_EC: return PADO_REG_M(4);
+    case RHS_ST_CE: return PADO_REG_M(5);
+    case RHS_ST_D1: return PADO_REG_M(6);
+    default: return PADO_REG_M(7);
     }
 #undef PADO_REG_M
 }

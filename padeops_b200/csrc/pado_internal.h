@@ -117,6 +117,10 @@ PADO_REG_PICK(0)
 PADO_REG_PICK(1)
 PADO_REG_PICK(2)
 PADO_REG_PICK(3)
+PADO_REG_PICK(4)
+PADO_REG_PICK(5)
+PADO_REG_PICK(6)
+PADO_REG_PICK(7)
 #undef PADO_REG_PICK
 RegFn pick_reg(int rk, int m, bool per, bool even, int mode, int lines);
 

@@ -9,17 +9,23 @@
 // row -- up to four groups coef * (m0 f[i0] + m1 f[i1] + ...), summed in order
 // -- that evaluates each row as the reference's array statement for it does
 // (same differences, same grouping), plus the factor table of its solve.
-// Device side: one thread per z line (lanes are consecutive x, so every row
-// access of a warp is one coalesced segment): forward sweep with the
-// right-hand side formed row by row, results through df, backward sweep.
+// Device side: lines of 24 points or more run in the register kernel
+// (pado_reg.cuh), whose end blocks take the closure rows from the row programs.
+// Shorter and uncuttable lines: one thread per z line (lanes are consecutive
+// x, so every row access of a warp is one coalesced segment), forward sweep
+// with the right-hand side formed row by row, results through df, backward
+// sweep: a serial chain of 2 n dependent row accesses.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cstring>
+#include <memory>
 #include <new>
 #include <vector>
 
 #include "pado_internal.h"
+
+using namespace pado;
 
 namespace {
 
@@ -39,6 +45,9 @@ struct StaggOp {
     int nin = 0, nout = 0, nsolve = 0;
     bool periodic = false, copy_first = false, valid = false;
     std::vector<SRow> rows;
+    std::vector<double> lower, diag, upper;  // non-periodic: the left-hand side
+    double alpha = 0.0, a = 0.0, b = 0.0, sign = 0.0;  // interior rows: band, taps (RegStagg)
+    std::unique_ptr<RegOp> reg;  // register kernel (null: the line does not cut)
     std::vector<double> fac;  // periodic: [nsolve][5] (bc, h, 1/c, a/c, v/c); else [nout][3] (ddn*den, den, cp)
     SRow *d_rows = nullptr;
     double *d_fac = nullptr;
@@ -141,6 +150,8 @@ struct pado_stagg_s {
     int n = 0, periodic = 1, top_even = 1, bot_even = 1, top_sided = 0, bot_sided = 0, device = 0;
     double dx = 1.0;
     StaggOp ops[PADO_STAGG_NOPS];
+    double *d_tab = nullptr;  // edge tables of every operator
+    int *d_status = nullptr;  // bounded waits of the register kernel
 };
 
 namespace {
@@ -240,13 +251,17 @@ void build_nonperiodic(pado_stagg_s *h)
     const bool te = h->top_even, be = h->bot_even, ts = h->top_sided, bs = h->bot_sided;
     const double odx = 1.0 / h->dx, odx2 = odx / h->dx;
     const C2CClosure C;
-    auto setop = [&](int k, int nin, int nout, const Builder &B, std::vector<double> fac) {
+    auto setop = [&](int k, int nin, int nout, const Builder &B, const std::vector<double> &ddn,
+                     const std::vector<double> &dg, const std::vector<double> &dup) {
         StaggOp &o = h->ops[k];
         o.nin = nin;
         o.nout = nout;
         o.nsolve = nout;
         o.rows = B.rows;
-        o.fac = std::move(fac);
+        o.fac = thomas(ddn, dg, dup);
+        o.lower = ddn;
+        o.diag = dg;
+        o.upper = dup;
         o.valid = true;
     };
     // ---- ddz_E2C (D1RHS_E2C_common.F90, ComputeTriD1_E2C) ----
@@ -299,7 +314,7 @@ void build_nonperiodic(pado_stagg_s *h)
         } else {
             ddn[0] = 0.0; dg[0] = be ? 1.0 - al : 1.0 + al;
         }
-        setop(PADO_STAGG_DDZ_E2C, nE, n, B, thomas(ddn, dg, dup));
+        setop(PADO_STAGG_DDZ_E2C, nE, n, B, ddn, dg, dup);
     }
     // ---- ddz_C2E (D1RHS_C2E_common.F90, ComputeTriD1_C2E) ----
     {
@@ -356,7 +371,7 @@ void build_nonperiodic(pado_stagg_s *h)
         } else {
             ddn[0] = 0.0; dup[0] = 2.0 * al;
         }
-        setop(PADO_STAGG_DDZ_C2E, n, nE, B, thomas(ddn, dg, dup));
+        setop(PADO_STAGG_DDZ_C2E, n, nE, B, ddn, dg, dup);
     }
     // ---- ddz_C2C (D1RHS_C2C_common.F90, ComputeTriD1_C2C) ----
     {
@@ -432,7 +447,7 @@ void build_nonperiodic(pado_stagg_s *h)
         } else {
             dg[0] = be ? 1.0 - al : 1.0 + al;
         }
-        setop(PADO_STAGG_DDZ_C2C, n, n, B, thomas(ddn, dg, dup));
+        setop(PADO_STAGG_DDZ_C2C, n, n, B, ddn, dg, dup);
     }
     // ---- ddz_E2E (D1RHS_E2E_common.F90, ComputeTriD1_E2E) ----
     {
@@ -463,7 +478,7 @@ void build_nonperiodic(pado_stagg_s *h)
         std::vector<double> ddn(nE, al), dg(nE, 1.0), dup(nE, al);
         dg[nE - 1] = 1.0; ddn[nE - 1] = te ? 0.0 : 2.0 * al;
         dg[0] = 1.0; dup[0] = be ? 0.0 : 2.0 * al;
-        setop(PADO_STAGG_DDZ_E2E, nE, nE, B, thomas(ddn, dg, dup));
+        setop(PADO_STAGG_DDZ_E2E, nE, nE, B, ddn, dg, dup);
     }
     // ---- d2dz2_C2C and d2dz2_E2E (D2RHS_*_common.F90, ComputeTriD2_*) ----
     for (int which = 0; which < 2; ++which) {
@@ -521,7 +536,7 @@ void build_nonperiodic(pado_stagg_s *h)
             dg[m - 1] = te ? 1.0 + al : 1.0 - al;
             dg[0] = be ? 1.0 + al : 1.0 - al;
         }
-        setop(e2e ? PADO_STAGG_D2DZ2_E2E : PADO_STAGG_D2DZ2_C2C, m, m, B, thomas(ddn, dg, dup));
+        setop(e2e ? PADO_STAGG_D2DZ2_E2E : PADO_STAGG_D2DZ2_C2C, m, m, B, ddn, dg, dup);
     }
     // ---- InterpZ_C2E (InterpRHS_C2E_common.F90, ComputeTriInterp_C2E) ----
     {
@@ -582,7 +597,7 @@ void build_nonperiodic(pado_stagg_s *h)
         } else {
             dup[0] = 0.0; dg[0] = 1.0;
         }
-        setop(PADO_STAGG_INTERPZ_C2E, n, nE, B, thomas(ddn, dg, dup));
+        setop(PADO_STAGG_INTERPZ_C2E, n, nE, B, ddn, dg, dup);
     }
     // ---- InterpZ_E2C (InterpRHS_E2C_common.F90, ComputeTriInterp_E2C) ----
     {
@@ -628,7 +643,7 @@ void build_nonperiodic(pado_stagg_s *h)
         } else {
             dg[0] = be ? 1.0 + al : 1.0 - al;
         }
-        setop(PADO_STAGG_INTERPZ_E2C, nE, n, B, thomas(ddn, dg, dup));
+        setop(PADO_STAGG_INTERPZ_E2C, nE, n, B, ddn, dg, dup);
     }
 }
 
@@ -704,8 +719,107 @@ __global__ void __launch_bounds__(256) stagg_kernel(const StaggLaunch p)
     if (p.copy_first) y[(long long)(p.nout - 1) * zs] = nxt;
 }
 
+// Interior rows of an operator: band and stencil.
+void interior(const pado_stagg_s *h, int k, StaggOp *o)
+{
+    const double odx = 1.0 / h->dx;
+    o->sign = k == PADO_STAGG_INTERPZ_E2C || k == PADO_STAGG_INTERPZ_C2E ? 1.0 : -1.0;
+    switch (k) {
+    case PADO_STAGG_DDZ_E2C:
+    case PADO_STAGG_DDZ_C2E:
+        o->alpha = 9.0 / 62.0;
+        o->a = (63.0 / 62.0) * odx;
+        o->b = ((17.0 / 62.0) / 3.0) * odx;
+        break;
+    case PADO_STAGG_DDZ_C2C:
+    case PADO_STAGG_DDZ_E2E:
+        o->alpha = 1.0 / 3.0;
+        o->a = (14.0 / 9.0) / 2.0 * odx;
+        o->b = (1.0 / 9.0) / 4.0 * odx;
+        break;
+    case PADO_STAGG_D2DZ2_C2C:
+    case PADO_STAGG_D2DZ2_E2E:
+        o->alpha = 2.0 / 11.0;
+        o->a = (12.0 / 11.0) * (h->periodic ? odx * odx : odx / h->dx);
+        o->b = (3.0 / 11.0) / 4.0 * (h->periodic ? odx * odx : odx / h->dx);
+        break;
+    default:
+        o->alpha = 3.0 / 10.0;
+        o->a = (3.0 / 2.0) / 2.0;
+        o->b = (1.0 / 10.0) / 2.0;
+    }
+}
+
+int stagg_rk(int k)
+{
+    switch (k) {
+    case PADO_STAGG_DDZ_E2C:
+    case PADO_STAGG_INTERPZ_E2C: return RHS_ST_EC;
+    case PADO_STAGG_DDZ_C2E:
+    case PADO_STAGG_INTERPZ_C2E: return RHS_ST_CE;
+    case PADO_STAGG_DDZ_C2C:
+    case PADO_STAGG_DDZ_E2E: return RHS_ST_D1;
+    default: return RHS_ST_D2;
+    }
+}
+
+// One closure row's program as the register kernel's groups on the 8 input
+// rows from `first`; false when it does not fit them.
+bool row_groups(const SRow &r, int first, double *out)
+{
+    bool single = r.ng > REG_GROUPS;  // a plain weighted sum written term by term: one group
+    if (single)
+        for (int g = 0; g < r.ng; ++g)
+            if (r.nt[g] != 1) return false;
+    for (int g = 0; g < r.ng; ++g) {
+        double *o = out + (single ? 0 : g) * 9;
+        o[0] = single ? 1.0 : r.coef[g];
+        for (int t = 0; t < r.nt[g]; ++t) {
+            const int j = r.idx[g][t] - first;
+            if (j < 0 || j > 7) return false;
+            o[1 + j] += single ? r.coef[g] * r.mul[g][t] : r.mul[g][t];
+        }
+    }
+    return true;
+}
+
+// The register kernel's constants of an operator, edge tables appended to
+// `all` from *off; null when its line does not cut into segments.
+std::unique_ptr<RegOp> stagg_reg(const StaggOp &o, std::vector<double> *all, size_t *off)
+{
+    if (o.nsolve < REG_MIN_N) return nullptr;
+    auto r = std::make_unique<RegOp>();
+    if (!choose_reg_cut(reg_rows(o.nsolve, o.periodic), false, &r->cut)) return nullptr;
+    RegStagg st;
+    st.n = o.nsolve;
+    st.nin = o.nin;
+    st.periodic = o.periodic;
+    st.copy_first = o.copy_first;
+    st.alpha = o.alpha;
+    st.a = o.a;
+    st.b = o.b;
+    st.sign = o.sign;
+    st.lower = o.lower.data();
+    st.diag = o.diag.data();
+    st.upper = o.upper.data();
+    for (int i = 0; i < 2 * REG_EDGE && !o.periodic; ++i) {
+        const int row = i < REG_EDGE ? i : o.nout - 2 * REG_EDGE + i;
+        if (!row_groups(o.rows[(size_t)row], i < REG_EDGE ? 0 : o.nin - 8, st.rows + i * REG_GROUPS * 9)) return nullptr;
+    }
+    std::memset(&r->kp, 0, sizeof(r->kp));
+    std::vector<double> tab;
+    reg_fill_stagg(st, r->cut, &r->kp, &tab);
+    *off = all->size();
+    all->insert(all->end(), tab.begin(), tab.end());
+    return r;
+}
+
 void free_ops(pado_stagg_s *h)
 {
+    if (h->d_tab) cudaFree(h->d_tab);
+    if (h->d_status) cudaFree(h->d_status);
+    h->d_tab = nullptr;
+    h->d_status = nullptr;
     for (auto &o : h->ops) {
         if (o.d_rows) cudaFree(o.d_rows);
         if (o.d_fac) cudaFree(o.d_fac);
@@ -729,6 +843,27 @@ int upload(pado_stagg_s *h)
             return pado::cuda_fail(e);
         }
     }
+    std::vector<double> all;
+    size_t off[PADO_STAGG_NOPS] = {0};
+    for (int k = 0; k < PADO_STAGG_NOPS; ++k) {
+        if (!h->ops[k].valid) continue;
+        interior(h, k, &h->ops[k]);
+        h->ops[k].reg = stagg_reg(h->ops[k], &all, &off[k]);
+    }
+    cudaError_t e = cudaMalloc(&h->d_status, sizeof(int));
+    if (e == cudaSuccess) e = cudaMemset(h->d_status, 0, sizeof(int));
+    if (e == cudaSuccess && !all.empty()) e = cudaMalloc(&h->d_tab, all.size() * sizeof(double));
+    if (e == cudaSuccess && !all.empty())
+        e = cudaMemcpy(h->d_tab, all.data(), all.size() * sizeof(double), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) {
+        free_ops(h);
+        return pado::cuda_fail(e);
+    }
+    for (int k = 0; k < PADO_STAGG_NOPS; ++k)
+        if (RegOp *r = h->ops[k].reg.get()) {
+            r->kp.segtab = h->d_tab ? h->d_tab + off[k] : nullptr;
+            r->kp.status = h->d_status;
+        }
     return PADO_OK;
 }
 
@@ -782,6 +917,14 @@ void pado_cd06stagg_destroy(pado_stagg_t stagg)
     delete stagg;
 }
 
+int pado_cd06stagg_status(pado_stagg_t stagg)
+{
+    if (!stagg) return PADO_E_NULL;
+    int v = 0;
+    const cudaError_t e = cudaMemcpy(&v, stagg->d_status, sizeof(int), cudaMemcpyDeviceToHost);
+    return e == cudaSuccess ? v : pado::cuda_fail(e);
+}
+
 int pado_cd06stagg_sizes(pado_stagg_t stagg, int op, int *nin, int *nout)
 {
     if (!stagg || !nin || !nout) return PADO_E_NULL;
@@ -804,6 +947,16 @@ int pado_cd06stagg_apply(pado_stagg_t stagg, int op, const double *f, double *df
     if (!f || !df) return PADO_E_NULL;
     const long long in_total = lines * o.nin, out_total = lines * o.nout;
     if (f < df + out_total && df < f + in_total) return PADO_E_ALIAS;
+    if (o.reg) {
+        RegLaunch r;
+        r.kp = o.reg->kp;
+        r.kp.in = f;
+        r.kp.out = df;
+        r.kp.nlines = r.kp.stride = lines;
+        r.kp.axis = 3;
+        // every line starts in the first plane: one row of n1 * n2 lines
+        if (plan_reg(stagg_rk(op), o.periodic, o.reg->cut, lines, 1, &r)) return launch_reg(r, (cudaStream_t)stream);
+    }
     StaggLaunch p;
     p.in = f;
     p.out = df;

@@ -67,6 +67,10 @@ class cd06stagg:  # noqa: N801 (reference name)
         check(L.lib().pado_cd06stagg_sizes(self._handle(), _OPS[name], ctypes.byref(nin), ctypes.byref(nout)), name)
         return nin.value, nout.value
 
+    def device_status(self) -> int:
+        """Status recorded by this object's kernels (0, or PADO_E_TIMEOUT)."""
+        return int(L.lib().pado_cd06stagg_status(self._handle()))
+
     def _handle(self) -> int:
         if not self._h.value:
             raise PadoError(L.E_STATE, "cd06stagg used before a successful init")

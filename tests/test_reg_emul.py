@@ -92,3 +92,58 @@ def test_register_kernel_other_system_emulated(emul):
         assert _run(emul, dense.CF90, dense.FILTER, n, 1.0, False, bc, (0, 0), 16, ROWS, 3, 0, 1.0, f, out) == 0
         ref = dense.apply_axis(D, f, 3)
         assert np.abs(out - ref).max() / np.abs(ref).max() <= 1e-12, bc
+
+
+# operator -> (RHS_ST_*, alpha, taps a, b, power of 1/dx, sign)
+STAGG = {"ddz_E2C": (4, 9 / 62, 63 / 62, 17 / 186, 1, -1), "ddz_C2E": (5, 9 / 62, 63 / 62, 17 / 186, 1, -1),
+         "InterpZ_E2C": (4, 0.3, 0.75, 0.05, 0, 1), "InterpZ_C2E": (5, 0.3, 0.75, 0.05, 0, 1),
+         "ddz_C2C": (6, 1 / 3, 7 / 9, 1 / 36, 1, -1), "ddz_E2E": (6, 1 / 3, 7 / 9, 1 / 36, 1, -1),
+         "d2dz2_C2C": (7, 2 / 11, 12 / 11, 3 / 44, 2, -1), "d2dz2_E2E": (7, 2 / 11, 12 / 11, 3 / 44, 2, -1)}
+
+
+@pytest.mark.parametrize("name", STAGG)
+@pytest.mark.parametrize("n", [24, 33, 64, 100])
+def test_staggered_operators_emulated(emul, name, n):
+    """The staggered operators' interior, end blocks (closure rows as one dense
+    group each, taken from the oracle's right-hand side of unit fields) and
+    cyclic wraps, against the oracle."""
+    from oracle.stagg import Stagg
+
+    rng = np.random.default_rng(n)
+    rk, alpha, a, b, order, sign = STAGG[name]
+    dx = 0.37
+    setups = [(True,)] if name not in ("ddz_C2C", "ddz_E2E") else []
+    setups += [(False, True, False, False, False), (False, False, True, False, False), (False, True, True, True, True)]
+    for setup in setups:
+        S = Stagg(n, dx, *setup)
+        op = S.OPS[name]
+        nin = n + 1 if name.split("_")[1].startswith("E") else n
+        nout = n + 1 if name.endswith("E") else n
+        f = rng.standard_normal((nin, 1, 13))
+        ref = S.apply(name, f)
+        rows = np.zeros((8, 3, 9))
+        if setup[0]:
+            lhs, solved = np.zeros((3, n)), n
+        else:
+            T = S.tri[op]  # lower / pivot, 1 / pivot, upper / pivot
+            lower, upper = T[:, 0] / T[:, 1], T[:, 2] / T[:, 1]
+            diag = 1 / T[:, 1] + np.concatenate([[0.0], lower[1:] * T[:-1, 2]])
+            lhs, solved = np.stack([lower, diag, upper]), nout
+            B = S._rhs_nonperiodic(op, np.eye(nin)[:, None, :])[:, 0, :]
+            rows[:, 0, 0] = 1.0
+            rows[:4, 0, 1:] = B[:4, :8]
+            rows[4:, 0, 1:] = B[-4:, -8:]
+        par = np.array([alpha, a / dx ** order, b / dx ** order, sign])
+        lhs = np.ascontiguousarray(lhs)
+        ran = 0
+        for m in (8, 16, 32):
+            out = np.full_like(ref, np.nan)
+            rc = emul.emul_reg_stagg(rk, solved, nin, int(setup[0]), int(setup[0] and nout > n), par.ctypes.data,
+                                     lhs.ctypes.data, rows.ctypes.data, m, f.ctypes.data, out.ctypes.data, 13)
+            if rc == -2:
+                continue
+            assert rc == 0
+            ran += 1
+            err = np.abs(out - ref).max() / np.abs(ref).max()
+            assert err <= 1e-12, (name, n, setup, m, err)
+        assert ran
