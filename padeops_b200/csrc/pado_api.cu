@@ -418,19 +418,19 @@ bool plan_stream(const pado_op_s *op, const DevTables &dt, const KParams &kp0, i
     return true;
 }
 
-bool plan_reg_op(const pado_op_s *op, const RegOp &ro, const KParams &kp0, int axis, long long na, long long nb, bool adj,
-                 RegLaunch *out)
+bool plan_reg_op(const pado_op_s *op, const RegOp &ro, int kind, int axis, const double *f, double *df, long long na,
+                 long long nb, bool adj, int out_mode, double out_alpha, RegLaunch *out)
 {
     RegParams &kp = out->kp;
     kp = ro.kp;
-    kp.in = kp0.in;
-    kp.out = kp0.out;
-    kp.nlines = kp0.nlines;
-    kp.stride = kp0.stride;
+    kp.in = f;
+    kp.out = df;
+    kp.nlines = na * nb;
+    kp.stride = axis == 1 ? 1 : (axis == 2 ? na : na * nb);
     kp.axis = axis;
-    kp.out_mode = kp0.out_mode;
-    kp.out_alpha = kp0.out_alpha;
-    const int rk = kp0.rc.rk;
+    kp.out_mode = out_mode;
+    kp.out_alpha = out_alpha;
+    const int rk = rhs_kind_of(op->scheme, kind);
     if (adj && (rk == RHS_CD06_D1 || rk == RHS_CD10_D1))
         for (double &t : kp.taps) t = -t;  // a cyclic first derivative is antisymmetric, the others symmetric
     return plan_reg(rk, op->periodic != 0, ro.cut, na, nb, out);
@@ -451,12 +451,18 @@ const RegOp *reg_op(const pado_op_s *op, int kind, int axis, const double *f, co
     return it == op->reg.end() ? nullptr : it->second.get();
 }
 
+// SMs of the current device, asked of the runtime once per device.
 int sm_count()
 {
+    constexpr int MAX_DEVICES = 64;
+    static std::atomic<int> known[MAX_DEVICES];
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
+    if (dev >= 0 && dev < MAX_DEVICES && (sms = known[dev].load(std::memory_order_relaxed)) > 0) return sms;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return sms > 0 ? sms : 1;
+    if (sms < 1) return 1;
+    if (dev >= 0 && dev < MAX_DEVICES) known[dev].store(sms, std::memory_order_relaxed);
+    return sms;
 }
 
 int launch_stream(pado_op_s *op, const StreamParams &sp, bool adj, int threads, size_t smem, int ctas_per_sm,
@@ -630,9 +636,9 @@ int launch_reg(const RegLaunch &r, cudaStream_t st)
 
 }  // namespace pado
 
-int pado::prepare_launch(pado_op_s *op, int kind, int axis, const double *f, double *df, long na, long nb, int bc1,
-                         int bcn, bool adjoint, int lines, bool no_fast, KParams *kpo, bool *trivial, int solve_bc1,
-                         int solve_bcn, int out_mode, double out_alpha)
+// Checks a request; *trivial: nothing for a line kernel to do.
+static int check_request(const pado_op_s *op, int kind, int axis, const double *f, const double *df, long na, long nb,
+                         int bc1, int bcn, bool *trivial)
 {
     *trivial = true;
     if (!op) return PADO_E_NULL;
@@ -646,7 +652,18 @@ int pado::prepare_launch(pado_op_s *op, int kind, int axis, const double *f, dou
     if (total == 0) return PADO_OK;
     if (!f || !df) return PADO_E_NULL;
     if (f < df + total && df < f + total) return PADO_E_ALIAS;
-    if (n == 1) return PADO_OK;
+    *trivial = n == 1;
+    return PADO_OK;
+}
+
+int pado::prepare_launch(pado_op_s *op, int kind, int axis, const double *f, double *df, long na, long nb, int bc1,
+                         int bcn, bool adjoint, int lines, bool no_fast, KParams *kpo, bool *trivial, int solve_bc1,
+                         int solve_bcn, int out_mode, double out_alpha)
+{
+    const int rc = check_request(op, kind, axis, f, df, na, nb, bc1, bcn, trivial);
+    if (rc != PADO_OK || *trivial) return rc;
+    *trivial = true;
+    const int n = op->n;
     const bool bounded_bc = !op->periodic && op->scheme != CD06;
     const int sb1 = solve_bc1 == SAME_BC ? bc1 : solve_bc1, sbn = solve_bcn == SAME_BC ? bcn : solve_bcn;
     auto it = op->tables.find(TabKey(kind, bounded_bc ? sb1 : 0, bounded_bc ? sbn : 0, adjoint ? 1 : 0));
@@ -696,10 +713,8 @@ int launch(pado_op_s *op, int kind, int axis, const double *f, double *df, long 
            double out_alpha = 1.0)
 {
     if (adjoint && out_mode != OUT_STORE) return PADO_E_UNSUPPORTED;
-    KParams kp;
     bool trivial = true;
-    int rc = prepare_launch(op, kind, axis, f, df, na, nb, bc1, bcn, adjoint, op ? op->lines : 0, false, &kp, &trivial,
-                            solve_bc1, solve_bcn, out_mode, out_alpha);
+    int rc = check_request(op, kind, axis, f, df, na, nb, bc1, bcn, &trivial);
     if (rc != PADO_OK) return rc;
     if (trivial) {
         const long long total = (long long)op->n * na * nb;
@@ -720,8 +735,12 @@ int launch(pado_op_s *op, int kind, int axis, const double *f, double *df, long 
     }
     if (const RegOp *ro = reg_op(op, kind, axis, f, df, bc1, bcn, adjoint, solve_bc1, solve_bcn)) {
         RegLaunch r;
-        if (plan_reg_op(op, *ro, kp, axis, na, nb, adjoint, &r)) return launch_reg(r, st);
+        if (plan_reg_op(op, *ro, kind, axis, f, df, na, nb, adjoint, out_mode, out_alpha, &r)) return launch_reg(r, st);
     }
+    KParams kp;
+    rc = prepare_launch(op, kind, axis, f, df, na, nb, bc1, bcn, adjoint, op->lines, false, &kp, &trivial, solve_bc1,
+                        solve_bcn, out_mode, out_alpha);
+    if (rc != PADO_OK) return rc;
     if (op->variant == 0 || op->variant == 4 || op->variant == 6) {
         const bool bounded_bc = !op->periodic && op->scheme != CD06;
         const int sb1 = solve_bc1 == SAME_BC ? bc1 : solve_bc1, sbn = solve_bcn == SAME_BC ? bcn : solve_bcn;
@@ -1113,7 +1132,7 @@ int pado_launch_plan(pado_op_t op, int kind, int axis, const double *f, double *
     if (rc != PADO_OK || trivial) return rc;
     if (const RegOp *ro = reg_op(op, kind, axis, f, df, bc1, bcn, false, SAME_BC, SAME_BC)) {
         RegLaunch r;
-        if (plan_reg_op(op, *ro, kp, axis, na, nb, false, &r)) {
+        if (plan_reg_op(op, *ro, kind, axis, f, df, na, nb, false, OUT_STORE, 1.0, &r)) {
             const bool copies = axis == 1 ? r.mode == REG_PACK : r.kp.async_copy != 0;
             info[0] = copies ? 6 : 4;
             info[1] = r.lines;
