@@ -105,7 +105,12 @@ void build_reg(pado_op_s *op, const std::vector<int> &kinds, const std::vector<s
         const RegKey key(kind, b1, bn, s1, sn, even_starts ? 1 : 0);
         if (op->reg.count(key)) return;
         auto r = std::make_unique<RegOp>();
-        if (!choose_reg_cut(reg_rows(n, op->periodic != 0), even_starts, &r->cut)) return;
+        // cyclic cf90 lines of up to 256 points: 16 rows, more threads to hide
+        // the longer link and close steps (GB/s along x / y / z, 32 -> 16 rows:
+        // n = 128 5539 / 5257 / 5195 -> 5905 / 6056 / 5911; n = 64 5466 / 5293 /
+        // 5237 -> 5269 / 5409 / 5332; bounded ones lose 10-25%)
+        const bool short_segments = op->scheme == CF90 && op->periodic && n <= 256;
+        if (!choose_reg_cut(reg_rows(n, op->periodic != 0), even_starts, short_segments, &r->cut)) return;
         std::memset(&r->kp, 0, sizeof(r->kp));
         std::vector<double> tab;
         const bool own = op->scheme == CD06;  // cd06 takes its closures from init (cd06.F90:177)
@@ -486,8 +491,9 @@ namespace pado {
 // link / close steps and the barriers per row of the next shorter one: 512
 // rows run 5-20% faster with 32 than with 16 (B200, all stencils and axes),
 // 64 to 128 rows within 5% of each other, 8 rows 10-50% slower.
-bool choose_reg_cut(int rows, bool even_starts, RegCut *cut)
+bool choose_reg_cut(int rows, bool even_starts, bool short_segments, RegCut *cut)
 {
+    if (short_segments && reg_cut(rows, 16, even_starts, cut)) return true;
     for (int M : {32, 16, 8})
         if (reg_cut(rows, M, even_starts, cut)) return true;
     return false;

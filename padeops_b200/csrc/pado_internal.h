@@ -132,7 +132,8 @@ struct RegLaunch {
     size_t smem = 0;
 };
 // The cut of a line of `rows` rows to cover into the longest segments it takes.
-bool choose_reg_cut(int rows, bool even_starts, RegCut *cut);
+// short_segments: 16 rows where it does.
+bool choose_reg_cut(int rows, bool even_starts, bool short_segments, RegCut *cut);
 // Plans the lines along `axis` of a field of the given geometry (out->kp: in,
 // out, nlines, stride, axis and output mode set on top of the operator's
 // constants); false when the field or line does not fit.

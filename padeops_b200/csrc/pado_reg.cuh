@@ -38,7 +38,7 @@
 // rounding of d and not that of f; f is added when d is complete.
 //
 // What bounds it: HBM, at 84-91% of the measured copy rate (6448 GB/s) for the
-// derivatives and 69-95% for cf90.  Per point the kernel issues the stencil (5
+// derivatives and 64-95% for cf90.  Per point the kernel issues the stencil (5
 // to 10 FP64), 4 recurrence and 4 correction FMAs, 1 + 2 H / M shared loads (H
 // the stencil's half width) and one store, against 67 to 90 instructions of
 // the streaming kernel, which keeps the line in shared memory and passes over
@@ -281,6 +281,12 @@ struct RegLine {
         t.xc.x = t.xc.y = 0.0;
 #pragma unroll
         for (int i = M - 1; i >= 0; --i) {
+#ifdef __CUDA_ARCH__
+            // no load of f moves up past here: all of the segment's would, and
+            // spill 25 registers (cf90 on 512^3, x + y + z: 1326 us with the
+            // spills, 1129 us without)
+            if (DIFF && (i + 1) % 8 == 0) __syncwarp(__activemask());
+#endif
             double d = t.x[i];
             if (!TRI && i < M - 2) d = fma(kp.np2, x2, d);
             if (i < M - 1) d = fma(kp.np1, x1, d);

@@ -789,7 +789,7 @@ std::unique_ptr<RegOp> stagg_reg(const StaggOp &o, std::vector<double> *all, siz
 {
     if (o.nsolve < REG_MIN_N) return nullptr;
     auto r = std::make_unique<RegOp>();
-    if (!choose_reg_cut(reg_rows(o.nsolve, o.periodic), false, &r->cut)) return nullptr;
+    if (!choose_reg_cut(reg_rows(o.nsolve, o.periodic), false, false, &r->cut)) return nullptr;
     RegStagg st;
     st.n = o.nsolve;
     st.nin = o.nin;
