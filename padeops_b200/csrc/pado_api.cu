@@ -435,6 +435,12 @@ bool plan_reg_op(const pado_op_s *op, const RegOp &ro, int kind, int axis, const
     kp.axis = axis;
     kp.out_mode = out_mode;
     kp.out_alpha = out_alpha;
+    if (axis == 3) {
+        // every z line starts in the first plane: one row of n1 n2 lines, tiles
+        // across the rows' ends (cd10 d1 on 33x997x256: 2950 -> 4200 GB/s)
+        na *= nb;
+        nb = 1;
+    }
     const int rk = rhs_kind_of(op->scheme, kind);
     if (adj && (rk == RHS_CD06_D1 || rk == RHS_CD10_D1))
         for (double &t : kp.taps) t = -t;  // a cyclic first derivative is antisymmetric, the others symmetric
@@ -561,6 +567,14 @@ bool plan_reg(int rk, bool per, const RegCut &cut, long long na, long long nb, R
     if (rk == RHS_CF90 && L * S > 256 && L > 16) L = 16;
     if (mode != REG_ROWS && L > 16) L = 16;
     if (mode == REG_SWZ && n > 128) L = 8;
+    // A strided tile's lines beyond the plane's edge are swept for nothing:
+    // fewer lines per tile where that fills 15% more of them (cd10 d1 along y,
+    // planes 33 wide: 2490 GB/s with 32 lines, 3550 with 8).
+    if (mode == REG_ROWS) {
+        auto swept = [&](int l) { return (na + l - 1) / l * l; };
+        for (int l = L / 2; l >= 8; l /= 2)
+            if (swept(L) * 20 > swept(l) * 23) L = l;
+    }
     int stages = mode == REG_SWZ ? 2 : 1;
     const int max_threads = M >= 32 ? 512 : 384;
     while (L > 8 && L * S > max_threads) L /= 2;
