@@ -551,16 +551,22 @@ struct RegOut {
             }
             return;
         }
+        // df's values (already on their way to L2, reg_prefetch) are read 8 rows ahead
         const bool acc = kp.out_mode == OUT_ACC;
+        double old[2][8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) old[0][i] = acc ? dst[i * kp.stride] : 0.0;
 #pragma unroll
         for (int c = 0; c < M; c += 8) {
-            double old[8];
+            if (c + 8 < M) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) old[i] = acc ? dst[(c + i) * kp.stride] : 0.0;
+                for (int i = 0; i < 8; ++i) old[(c / 8 + 1) & 1][i] = acc ? dst[(c + 8 + i) * kp.stride] : 0.0;
+            }
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 const double x = RL::corrected(kp, t, c + i, t.x[c + i]);
-                if (EVEN || c + i >= REG_OVERLAP || c + i >= op) dst[(c + i) * kp.stride] = fma(kp.out_alpha, x, old[i]);
+                if (EVEN || c + i >= REG_OVERLAP || c + i >= op)
+                    dst[(c + i) * kp.stride] = fma(kp.out_alpha, x, old[(c / 8) & 1][i]);
             }
         }
     }
@@ -812,6 +818,31 @@ __device__ __forceinline__ void reg_load_async(const RegParams &kp, double *tile
     async_arrive(bar);
 }
 
+// Accumulated output: tile t's part of df on its way to L2 while the tile's
+// copies are, so that out() does not wait for HBM (divergence + laplacian on
+// 384x256x192: 541 -> 525 us; with the reads 8 rows ahead of their use in
+// RegOut::rows 515 us).
+template <int MODE, int LT>
+__device__ __forceinline__ void reg_prefetch(const RegParams &kp, long long t, int tid, int nthreads)
+{
+    long long x0, p;
+    reg_origin(kp, LT, t, &x0, &p);
+    if constexpr (MODE == REG_ROWS) {
+        constexpr int LINE = LT < 16 ? LT : 16, PER_ROW = LT / LINE;  // 128 bytes
+        const int total = kp.n * PER_ROW;
+        for (int i = tid; i < total; i += nthreads) {
+            const int r = i / PER_ROW, c = (i % PER_ROW) * LINE;
+            if (x0 + c < kp.na)
+                asm volatile("prefetch.global.L2 [%0];\n" ::"l"(kp.out + x0 + c + p * kp.pstride + r * kp.stride));
+        }
+    } else {
+        const long long left = kp.nlines - x0;
+        const int total = (int)(left < LT ? left : LT) * kp.n;
+        for (int i = tid * 16; i < total; i += nthreads * 16)
+            asm volatile("prefetch.global.L2 [%0];\n" ::"l"(kp.out + x0 * (long long)kp.n + i));
+    }
+}
+
 // Registers: a segment of 32 rows takes 64 for its values and about 45 more,
 // so 512 threads fill an SM; shorter segments leave room for more threads.
 template <int M>
@@ -857,6 +888,8 @@ __global__ void __launch_bounds__(RegBounds<M>::threads, RegBounds<M>::ctas) reg
                 reg_load<MODE, LT>(kp, base + (size_t)b * kp.tile_doubles, &bars[b], blockIdx.x + b * G);
     }
 
+    const bool acc = kp.out_mode == OUT_ACC;
+    if (acc && blockIdx.x < kp.ntiles) reg_prefetch<MODE, LT>(kp, blockIdx.x, tid, nthreads);
     int b = 0;
     unsigned parity = 0;
     for (long long t = blockIdx.x; t < kp.ntiles; t += G) {
@@ -893,6 +926,7 @@ __global__ void __launch_bounds__(RegBounds<M>::threads, RegBounds<M>::ctas) reg
                 reg_load<MODE, LT>(kp, base + (size_t)(b ^ 1) * kp.tile_doubles, &bars[b ^ 1], t + G);
             }
         }
+        if (acc && t + G < kp.ntiles) reg_prefetch<MODE, LT>(kp, t + G, tid, nthreads);
         if (active) PH::link(kp, sm, th, l, s);
         __syncthreads();
         if (active) PH::close(kp, sm, th, l, s);
