@@ -552,7 +552,16 @@ bool plan_reg(int rk, bool per, const RegCut &cut, long long na, long long nb, R
     if (align_bits & 7) return false;
     const bool xl = axis == 1;
     const bool tma_ok = !(align_bits & 15) && (xl ? n % 2 == 0 : na % 2 == 0);
-    const int mode = xl ? (tma_ok ? REG_SWZ : REG_PACK) : REG_ROWS;
+    // strided lines an odd number of elements apart: rows of one parity are
+    // 16-byte aligned, so each has its own tensor copy (the output takes plain
+    // stores); x lines of odd extent: a tile's span is whole 16-byte units.
+    // Against 8-byte copies by every thread (GB/s, x / y / z of 511 rows, planes
+    // 511 wide): cd10 d1 cyclic 4433 / 4600 / 4378 -> 5792 / 5589 / 5408, bounded
+    // 4202 / 4254 / 4099 -> 5369 / 5118 / 5088.
+    const bool odd = !xl && na % 2 && (axis == 2 || nb == 1) && !(reinterpret_cast<size_t>(kp.in) & 15) &&
+                     na * (nb * nin) <= 0x7fffffffLL;
+    const bool span = xl && n % 2 && !(align_bits & 15);
+    const int mode = xl ? (tma_ok ? REG_SWZ : REG_PACK) : (odd ? REG_ODD : REG_ROWS);
     const bool even = per && cut.even();
     // Lines per tile, measured on 2^25..2^26 points (GB/s).  Strided lines: as
     // many as 512 threads sweep (longer rows for the copy engine and DRAM:
@@ -565,17 +574,18 @@ bool plan_reg(int rk, bool per, const RegCut &cut, long long na, long long nb, R
     // 64 bounded: 4490 against 3490).
     int L = S * 32 <= 512 ? 32 : (S * 16 <= 512 ? 16 : 8);
     if (rk == RHS_CF90 && L * S > 256 && L > 16) L = 16;
-    if (mode != REG_ROWS && L > 16) L = 16;
+    if (xl && L > 16) L = 16;
     if (mode == REG_SWZ && n > 128) L = 8;
     // A strided tile's lines beyond the plane's edge are swept for nothing:
     // fewer lines per tile where that fills 15% more of them (cd10 d1 along y,
     // planes 33 wide: 2490 GB/s with 32 lines, 3550 with 8).
-    if (mode == REG_ROWS) {
+    if (!xl) {
         auto swept = [&](int l) { return (na + l - 1) / l * l; };
         for (int l = L / 2; l >= 8; l /= 2)
             if (swept(L) * 20 > swept(l) * 23) L = l;
     }
-    int stages = mode == REG_SWZ ? 2 : 1;
+    int stages = mode == REG_SWZ || span ? 2 : 1;
+    kp.async_copy = mode == REG_PACK && !span ? 1 : 0;
     const int max_threads = M >= 32 ? 512 : 384;
     while (L > 8 && L * S > max_threads) L /= 2;
     const int threads = (L * S + 31) / 32 * 32;
@@ -591,10 +601,12 @@ bool plan_reg(int rk, bool per, const RegCut &cut, long long na, long long nb, R
         kp.xblocks = (int)((na + L - 1) / L);
         kp.ntiles = (long long)kp.xblocks * nb;
         kp.pstride = axis == 2 ? na * (long long)nin : na;
-        kp.async_copy = tma_ok ? 0 : 1;
-        kp.nbox = (nin + 255) / 256;
-        kp.box_rows = ((nin + kp.nbox - 1) / kp.nbox + 15) / 16 * 16;
-        kp.tile_doubles = (tma_ok ? kp.nbox * kp.box_rows : (nin + 15) / 16 * 16) * L;
+        kp.async_copy = tma_ok || odd ? 0 : 1;
+        const int rows = odd ? (nin + 1) / 2 : nin;  // rows a map takes of a tile
+        kp.nbox = (rows + 255) / 256;
+        kp.box_rows = ((rows + kp.nbox - 1) / kp.nbox + 15) / 16 * 16;
+        kp.odd_rows = kp.nbox * kp.box_rows * (L + 2);
+        kp.tile_doubles = odd ? 2 * kp.odd_rows : (tma_ok ? kp.nbox * kp.box_rows : (nin + 15) / 16 * 16) * L;
     }
     if (kp.ntiles > 0x7fffffffLL) return false;
     const int edge_table = reg_edge_table(rk, per, S);
@@ -608,7 +620,7 @@ bool plan_reg(int rk, bool per, const RegCut &cut, long long na, long long nb, R
     if (!grant_smem((const void *)out->fn)) return false;
     const int ctas = resident_ctas((const void *)out->fn, threads, out->smem);
     if (ctas < 1) return false;
-    if (tma_ok) {
+    if (tma_ok || odd) {
         EncodeTiledFn enc = encode_tiled();
         if (!enc) return false;
         auto map = [&](CUtensorMap *m, const double *p, int rank, const cuuint64_t *dims, const cuuint64_t *strides,
@@ -628,6 +640,16 @@ bool plan_reg(int rk, bool per, const RegCut &cut, long long na, long long nb, R
             const cuuint32_t b2[2] = {16, (cuuint32_t)L};
             if (n % 16 && !(map(&kp.tin2, kp.in, 2, d2, s2, b2, CU_TENSOR_MAP_SWIZZLE_128B) &&
                             map(&kp.tout2, kp.out, 2, d2, s2, b2, CU_TENSOR_MAP_SWIZZLE_128B)))
+                return false;
+        } else if (odd) {
+            // rows of the whole field, na apart: even ones from the start, odd ones from the element before theirs
+            const long long rows = axis == 2 ? nb * nin : nin, step = axis == 2 ? na : na * nb;
+            const cuuint64_t stride[1] = {(cuuint64_t)step * 16};
+            const cuuint64_t de[2] = {(cuuint64_t)na, (cuuint64_t)((rows + 1) / 2)};
+            const cuuint64_t dodd[2] = {(cuuint64_t)na + 1, (cuuint64_t)(rows / 2)};
+            const cuuint32_t box[2] = {(cuuint32_t)L + 2, (cuuint32_t)kp.box_rows};
+            if (!map(&kp.tin, kp.in, 2, de, stride, box, CU_TENSOR_MAP_SWIZZLE_NONE) ||
+                !map(&kp.tin2, kp.in + step - 1, 2, dodd, stride, box, CU_TENSOR_MAP_SWIZZLE_NONE))
                 return false;
         } else {
             const cuuint64_t dims[3] = {(cuuint64_t)na, (cuuint64_t)(axis == 2 ? nin : nb), (cuuint64_t)(axis == 2 ? nb : nin)};
@@ -1153,7 +1175,7 @@ int pado_launch_plan(pado_op_t op, int kind, int axis, const double *f, double *
     if (const RegOp *ro = reg_op(op, kind, axis, f, df, bc1, bcn, false, SAME_BC, SAME_BC)) {
         RegLaunch r;
         if (plan_reg_op(op, *ro, kind, axis, f, df, na, nb, false, OUT_STORE, 1.0, &r)) {
-            const bool copies = axis == 1 ? r.mode == REG_PACK : r.kp.async_copy != 0;
+            const bool copies = r.mode == REG_PACK || r.mode == REG_ODD || r.kp.async_copy;
             info[0] = copies ? 6 : 4;
             info[1] = r.lines;
             info[2] = r.kp.stages;

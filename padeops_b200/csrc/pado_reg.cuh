@@ -75,8 +75,13 @@ PADO_HD constexpr int reg_edge_table(int rk, bool periodic, int S)
 enum RegMode {
     REG_ROWS = 0,   // strided lines: [row][L] tile (tensor copies, or per-element copies); results stored from registers
     REG_SWZ = 1,    // x lines: 16-row chunks [chunk][L][16] with the 128-byte swizzle, tensor copies in and out
-    REG_PACK = 2    // x lines of any extent and alignment: [L][P], P odd, per-element copies
+    REG_ODD = 3,    // strided lines an odd number of elements apart: as REG_ROWS, the tile's even and odd rows copied
+                    // apart (each 16-byte aligned), [2][rows][L + 2]
+    REG_PACK = 2    // x lines of odd extent: [L][n], one bulk copy of the tile's span in and out; of any extent and
+                    // alignment (async_copy): [L][P], P odd, per-element copies
 };
+
+PADO_HD constexpr bool reg_strided(int mode) { return mode == REG_ROWS || mode == REG_ODD; }
 
 struct alignas(64) RegParams {
     CUtensorMap tin, tout;      // tensor copies (x lines: whole 16-row chunks)
@@ -90,8 +95,9 @@ struct alignas(64) RegParams {
     int n, S, W, na, xblocks, axis, out_mode;
     int nin;                    // rows of the input (n but for the staggered scheme's cells and edges)
     int copy_first;             // the result's last row repeats its first (cyclic edges)
-    int async_copy;             // REG_ROWS: per-element copies
+    int async_copy;             // REG_ROWS, REG_PACK: per-element copies
     int chunks;                 // REG_SWZ: whole chunks per line
+    int odd_rows;               // REG_ODD: doubles from the even rows' part of a tile to the odd rows'
     int stages, tile_doubles, nbox, box_rows, P;
     int d0, d1, nd1;            // overlap at joint j (between segments j - 1 and j): d1 for 1 <= j <= nd1, else d0
     int cyc;                    // cyclic lines: the states pass round the line more than once (wrap)
@@ -136,6 +142,7 @@ PADO_HD PADO_INLINE size_t reg_smem_bytes(int L, int S, int stages, int tile_dou
 
 struct RegSmem {
     double *tile;   // the buffer of this tile
+    int first;      // REG_ODD: parity of the tile's first row in the field
     double2 *ys;    // [S][L] y state each segment hands on
     double2 *xs;    // [S][L] x state each segment hands back
     double *edge;   // [REG_EDGE_DOUBLES][L]
@@ -164,6 +171,35 @@ struct RowsAt {
     PADO_HD PADO_INLINE double get(int k) const
     {
         return k < LOW ? lo[k * RS] : (k < M + HIGH ? p[k * RS] : hi[k * RS]);
+    }
+};
+
+// The same where a tile's rows of either parity lie apart (REG_ODD): rows r of
+// the tile at par[r & 1] + (r >> 1) (LT + 2).
+template <int LT, int RK>
+struct OddAt {
+    static constexpr int RS = LT + 2;
+    static constexpr int SHIFT = RowsAt<1, RK>::SHIFT, LOW = RowsAt<1, RK>::LOW, HIGH = RowsAt<1, RK>::HIGH;
+    const double *p[2], *lo[2], *hi[2];  // rows of even and odd k
+    PADO_HD PADO_INLINE static const double *place(const double *const (&par)[2], int r)
+    {
+        return par[r & 1] + (r >> 1) * RS;  // r may be negative: floor
+    }
+    PADO_HD PADO_INLINE OddAt(const double *const (&par)[2], int n, int start, int m, bool cyclic)
+    {
+        const int r = start + SHIFT, rl = cyclic && start == 0 ? r + n : r, rh = cyclic && start + m == n ? r - n : r;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            p[k] = place(par, r + k);
+            lo[k] = place(par, rl + k);
+            hi[k] = place(par, rh + k);
+        }
+    }
+    template <int M>
+    PADO_HD PADO_INLINE double get(int k) const
+    {
+        const double *const(&b)[2] = k < LOW ? lo : (k < M + HIGH ? p : hi);
+        return b[k & 1][(k >> 1) * RS];
     }
 };
 
@@ -607,7 +643,7 @@ struct RegOut {
     {
 #pragma unroll
         for (int i = 0; i < REG_EDGE; ++i) {
-            if constexpr (MODE == REG_ROWS) {
+            if constexpr (reg_strided(MODE)) {
                 double *d = line + (row0 + i) * kp.stride;
                 if (live) *d = kp.out_mode == OUT_ACC ? fma(kp.out_alpha, e[i], *d)
                                                       : (kp.out_mode == OUT_SCALE ? kp.out_alpha * e[i] : e[i]);
@@ -647,6 +683,16 @@ struct RegPhases {
                 return i & 1 ? pair.y : pair.x;
             };
             RL::sweep(kp, t, od, op, load, again, last);
+        } else if constexpr (MODE == REG_ODD) {
+            const double *par[2];
+            parities(kp, sm, l, par);
+            const OddAt<LT, RK> at(par, kp.n, st, M, PER);
+            auto load = [&](double(&f)[M + 2 * H]) {
+#pragma unroll
+                for (int k = -H; k < M + H; ++k) f[k + H] = at.template get<M>(k);
+            };
+            auto again = [&](int i) { return at.template get<M>(i); };
+            RL::sweep(kp, t, od, op, load, again, last);
         } else {
             constexpr int RS = MODE == REG_ROWS ? LT : 1;
             const RowsAt<RS, RK> at(MODE == REG_ROWS ? sm.tile + l : sm.tile + (long long)l * kp.P, kp.n, st, M, PER);
@@ -676,9 +722,20 @@ struct RegPhases {
             }
         }
     }
+    // REG_ODD: rows 0 and 1 of line l (odd rows of the field sit one element further in)
+    PADO_HD PADO_INLINE static void parities(const RegParams &kp, const RegSmem &sm, int l, const double *(&par)[2])
+    {
+        const double *even = sm.tile + l, *odd = sm.tile + kp.odd_rows + l + 1;
+        par[0] = sm.first ? odd : even;
+        par[1] = sm.first ? even : odd;
+    }
     PADO_HD PADO_INLINE static double row(const RegParams &kp, const RegSmem &sm, int l, int r)
     {
-        if constexpr (MODE == REG_ROWS) return sm.tile[r * LT + l];
+        if constexpr (MODE == REG_ODD) {
+            const double *par[2];
+            parities(kp, sm, l, par);
+            return *OddAt<LT, RK>::place(par, r);
+        } else if constexpr (MODE == REG_ROWS) return sm.tile[r * LT + l];
         else return *RO::at(kp, sm.tile, l, r);
     }
     PADO_HD PADO_INLINE static double2 last_rows(const RegSmem &sm, int l)
@@ -718,7 +775,7 @@ struct RegPhases {
                 RO::edge(kp, sm, e, l, kp.n - REG_EDGE, dst, live);
             }
         }
-        if constexpr (MODE == REG_ROWS) {
+        if constexpr (reg_strided(MODE)) {
             if (live) RO::rows(kp, t, dst + st * kp.stride, op);
             if constexpr (PER && (RK == RHS_ST_CE || RK == RHS_ST_D2))
                 if (live && s == 0 && kp.copy_first) dst[kp.n * kp.stride] = RL::corrected(kp, t, 0, t.x[0]);
@@ -750,7 +807,15 @@ __device__ __forceinline__ void tma_store_3d(const CUtensorMap *map, const void 
                  : "memory");
 }
 
-// Tensor copies of tile t into `tile` (one thread).
+// Elements of the x-line tile from line x0.
+template <int LT>
+__device__ __forceinline__ int reg_span(const RegParams &kp, long long x0)
+{
+    const long long left = kp.nlines - x0;
+    return (int)(left < LT ? left : LT) * kp.n;
+}
+
+// Tensor or bulk copies of tile t into `tile` (one thread).
 template <int MODE, int LT>
 __device__ __forceinline__ void reg_load(const RegParams &kp, double *tile, unsigned long long *bar, long long t)
 {
@@ -761,6 +826,20 @@ __device__ __forceinline__ void reg_load(const RegParams &kp, double *tile, unsi
         mbar_expect_tx(bar, (unsigned)(kp.chunks + (part ? 1 : 0)) * LT * 128u);
         if (kp.chunks) tma_load_3d(tile, &kp.tin, bar, 0, (int)x0, 0);
         if (part) tma_load_2d(tile + (size_t)kp.chunks * LT * 16, &kp.tin2, bar, kp.chunks * 16, (int)x0);
+    } else if constexpr (MODE == REG_ODD) {
+        // rows p nin .. p nin + nin - 1 of the field, those of either parity from their own map
+        const int r0 = kp.axis == 2 ? (int)p * kp.nin : 0;
+        mbar_expect_tx(bar, 2u * kp.nbox * kp.box_rows * (LT + 2) * 8u);
+        for (int b = 0; b < kp.nbox; ++b) {
+            double *dst = tile + (size_t)b * kp.box_rows * (LT + 2);
+            tma_load_2d(dst, &kp.tin, bar, (int)x0, ((r0 + 1) >> 1) + b * kp.box_rows);
+            tma_load_2d(dst + kp.odd_rows, &kp.tin2, bar, (int)x0, (r0 >> 1) + b * kp.box_rows);
+        }
+    } else if constexpr (MODE == REG_PACK) {
+        // whole 16-byte units of the span (tiles start on them: LT is even)
+        const unsigned bytes = ((unsigned)reg_span<LT>(kp, x0) * 8u) & ~15u;
+        mbar_expect_tx(bar, bytes);
+        bulk_load(tile, kp.in + x0 * (long long)kp.n, bytes, bar);
     } else {
         mbar_expect_tx(bar, (unsigned)kp.nbox * kp.box_rows * LT * 8u);
         for (int b = 0; b < kp.nbox; ++b) {
@@ -827,7 +906,7 @@ __device__ __forceinline__ void reg_prefetch(const RegParams &kp, long long t, i
 {
     long long x0, p;
     reg_origin(kp, LT, t, &x0, &p);
-    if constexpr (MODE == REG_ROWS) {
+    if constexpr (reg_strided(MODE)) {
         constexpr int LINE = LT < 16 ? LT : 16, PER_ROW = LT / LINE;  // 128 bytes
         const int total = kp.n * PER_ROW;
         for (int i = tid; i < total; i += nthreads) {
@@ -858,7 +937,7 @@ __global__ void __launch_bounds__(RegBounds<M>::threads, RegBounds<M>::ctas) reg
     using RO = RegOut<RK, PER, M, EVEN, MODE, LT>;
     extern __shared__ double smem_raw[];
     double *base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u) / sizeof(double);
-    const int S = kp.S, stages = MODE == REG_SWZ ? kp.stages : 1;
+    const int S = kp.S, stages = reg_strided(MODE) ? 1 : kp.stages;
     const int edge_table = reg_edge_table(RK, PER, S);
     const RegLayout lay = reg_layout(LT, S, stages, kp.tile_doubles, edge_table);
     unsigned long long *bars = reinterpret_cast<unsigned long long *>(base + lay.bars);
@@ -870,7 +949,7 @@ __global__ void __launch_bounds__(RegBounds<M>::threads, RegBounds<M>::ctas) reg
     const int tid = threadIdx.x, nthreads = blockDim.x;
     const int l = tid % LT, s = tid / LT;
     const bool active = s < S;
-    const bool async = MODE == REG_PACK || (MODE == REG_ROWS && kp.async_copy);
+    const bool async = (MODE == REG_ROWS || MODE == REG_PACK) && kp.async_copy;
     const long long G = gridDim.x;
 
     if (tid == 0) {
@@ -893,6 +972,14 @@ __global__ void __launch_bounds__(RegBounds<M>::threads, RegBounds<M>::ctas) reg
     int b = 0;
     unsigned parity = 0;
     for (long long t = blockIdx.x; t < kp.ntiles; t += G) {
+        if (MODE == REG_PACK && !async && tid == nthreads - 1) {
+            // a last tile of an odd number of elements: the one past its whole units
+            long long x0, p;
+            reg_origin(kp, LT, t, &x0, &p);
+            const int total = reg_span<LT>(kp, x0);
+            if (total & 1)
+                base[(size_t)b * kp.tile_doubles + total - 1] = __ldg(kp.in + x0 * (long long)kp.n + total - 1);
+        }
         bool arrived = true;
         if (tid < 32) arrived = mbar_wait(&bars[b], parity, STREAM_WAIT_NS);
         if (!__syncthreads_and(arrived)) {
@@ -904,23 +991,24 @@ __global__ void __launch_bounds__(RegBounds<M>::threads, RegBounds<M>::ctas) reg
                     (void)mbar_wait(&bars[b ^ 1], b ? parity ^ 1u : parity, STREAM_DRAIN_NS);
             }
             if (async) async_wait_all();
-            else if (MODE == REG_SWZ) bulk_wait_all();
+            else if (!reg_strided(MODE)) bulk_wait_all();
             return;
         }
         sm.tile = base + (size_t)b * kp.tile_doubles;
         long long x0, p;
         reg_origin(kp, LT, t, &x0, &p);
+        sm.first = MODE == REG_ODD && kp.axis == 2 ? (int)(p * kp.nin & 1) : 0;
         RegThread<M> th;
         if (active) PH::sweep(kp, sm, th, l, s);
         __syncthreads();
         // every read of the tile is done: strided lines take the next one now,
         // x lines their other buffer, once its results have been read out
-        if constexpr (MODE == REG_ROWS) {
+        if constexpr (reg_strided(MODE)) {
             if (t + G < kp.ntiles) {
                 if (async) reg_load_async<MODE, LT>(kp, sm.tile, &bars[0], t + G, tid, nthreads);
                 else if (tid == 0) reg_load<MODE, LT>(kp, sm.tile, &bars[0], t + G);
             }
-        } else if constexpr (MODE == REG_SWZ) {
+        } else {
             if (stages == 2 && tid == 0 && t != blockIdx.x && t + G < kp.ntiles) {
                 bulk_wait_read();
                 reg_load<MODE, LT>(kp, base + (size_t)(b ^ 1) * kp.tile_doubles, &bars[b ^ 1], t + G);
@@ -931,46 +1019,59 @@ __global__ void __launch_bounds__(RegBounds<M>::threads, RegBounds<M>::ctas) reg
         __syncthreads();
         if (active) PH::close(kp, sm, th, l, s);
         if constexpr (!PER) __syncthreads();
-        const bool live = MODE != REG_ROWS || x0 + l < kp.na;
-        double *dst = MODE == REG_ROWS ? kp.out + (live ? x0 + l + p * kp.pstride : 0) : nullptr;
+        const bool live = !reg_strided(MODE) || x0 + l < kp.na;
+        double *dst = reg_strided(MODE) ? kp.out + (live ? x0 + l + p * kp.pstride : 0) : nullptr;
         if (active) PH::out(kp, sm, th, l, s, dst, live);
-        if constexpr (MODE != REG_ROWS) {
+        if constexpr (!reg_strided(MODE)) {
             const long long left = kp.nlines - x0;
             const int nl = (int)(left < LT ? left : LT), n = kp.n;
-            if (MODE == REG_SWZ && kp.out_mode != OUT_STORE) {
-                // scaled or accumulated output: df's values, two rows at a time
+            if (!async && kp.out_mode != OUT_STORE) {
+                // scaled or accumulated output: the tile takes df's values before it goes out
                 __syncthreads();
-                const int half = n >> 1, warp = tid >> 5, lane = tid & 31, nw = nthreads >> 5;
-                for (int ll = warp; ll < nl; ll += nw) {
-                    const double2 *d = reinterpret_cast<const double2 *>(kp.out + (x0 + ll) * (long long)n);
-                    for (int u = lane; u < half; u += 32) {
-                        double2 *x = reinterpret_cast<double2 *>(RO::at(kp, sm.tile, ll, 2 * u));
-                        double2 v = *x;
-                        if (kp.out_mode == OUT_ACC) {
-                            const double2 o = d[u];
-                            v.x = fma(kp.out_alpha, v.x, o.x);
-                            v.y = fma(kp.out_alpha, v.y, o.y);
-                        } else {
-                            v.x *= kp.out_alpha;
-                            v.y *= kp.out_alpha;
+                if constexpr (MODE == REG_SWZ) {
+                    const int half = n >> 1, warp = tid >> 5, lane = tid & 31, nw = nthreads >> 5;
+                    for (int ll = warp; ll < nl; ll += nw) {
+                        const double2 *d = reinterpret_cast<const double2 *>(kp.out + (x0 + ll) * (long long)n);
+                        for (int u = lane; u < half; u += 32) {
+                            double2 *x = reinterpret_cast<double2 *>(RO::at(kp, sm.tile, ll, 2 * u));
+                            double2 v = *x;
+                            if (kp.out_mode == OUT_ACC) {
+                                const double2 o = d[u];
+                                v.x = fma(kp.out_alpha, v.x, o.x);
+                                v.y = fma(kp.out_alpha, v.y, o.y);
+                            } else {
+                                v.x *= kp.out_alpha;
+                                v.y *= kp.out_alpha;
+                            }
+                            *x = v;
                         }
-                        *x = v;
                     }
+                } else {
+                    const double *d = kp.out + x0 * (long long)n;
+                    for (int e = tid; e < nl * n; e += nthreads)
+                        sm.tile[e] = kp.out_mode == OUT_ACC ? fma(kp.out_alpha, sm.tile[e], d[e]) : kp.out_alpha * sm.tile[e];
                 }
             }
-            if constexpr (MODE == REG_SWZ) {
+            if (!async) {
                 fence_proxy_async();
                 __syncthreads();
                 if (tid == 0) {
-                    if (kp.chunks) tma_store_3d(&kp.tout, sm.tile, 0, (int)x0, 0);
-                    if (n & 15) tma_store_2d(&kp.tout2, sm.tile + (size_t)kp.chunks * LT * 16, kp.chunks * 16, (int)x0);
+                    if constexpr (MODE == REG_SWZ) {
+                        if (kp.chunks) tma_store_3d(&kp.tout, sm.tile, 0, (int)x0, 0);
+                        if (n & 15) tma_store_2d(&kp.tout2, sm.tile + (size_t)kp.chunks * LT * 16, kp.chunks * 16, (int)x0);
+                    } else {
+                        const int total = nl * n;
+                        double *d = kp.out + x0 * (long long)n;
+                        bulk_store(d, sm.tile, ((unsigned)total * 8u) & ~15u);
+                        if (total & 1) d[total - 1] = sm.tile[total - 1];
+                    }
                     bulk_commit();
                     if (stages == 1) {
                         bulk_wait_read();
                         if (t + G < kp.ntiles) reg_load<MODE, LT>(kp, sm.tile, &bars[0], t + G);
                     }
                 }
-            } else {
+            } else if constexpr (MODE == REG_PACK) {
                 // the tile's lines are consecutive in global memory
                 __syncthreads();
                 const int pad = kp.P - n, total = nl * n;
@@ -1002,7 +1103,7 @@ __global__ void __launch_bounds__(RegBounds<M>::threads, RegBounds<M>::ctas) reg
             parity ^= 1u;
         }
     }
-    if (MODE == REG_SWZ) bulk_wait_all();
+    if (!reg_strided(MODE) && !async) bulk_wait_all();
 }
 #endif  // __CUDACC__
 
@@ -1030,22 +1131,26 @@ inline void emulate_reg(const RegParams &kp)
         long long x0, p;
         reg_origin(kp, LT, t, &x0, &p);
         const long long lim = kp.axis == 1 ? kp.nlines : kp.na;
+        sm.first = MODE == REG_ODD && kp.axis == 2 ? (int)(p * kp.nin & 1) : 0;
         for (int l = 0; l < LT && x0 + l < lim; ++l)
             for (int r = 0; r < kp.nin; ++r) {
                 if (MODE == REG_ROWS) sm.tile[r * LT + l] = kp.in[x0 + l + p * kp.pstride + r * kp.stride];
+                else if (MODE == REG_ODD)
+                    sm.tile[((sm.first + r) & 1 ? kp.odd_rows + 1 : 0) + (r >> 1) * (LT + 2) + l] =
+                        kp.in[x0 + l + p * kp.pstride + r * kp.stride];
                 else *RO::at(kp, sm.tile, l, r) = kp.in[(x0 + l) * kp.n + r];
             }
         for (int ph = 0; ph < 4; ++ph)
             for (int s = 0; s < kp.S; ++s)
                 for (int l = 0; l < LT; ++l) {
                     RegThread<M> &h = th[(size_t)s * LT + l];
-                    const bool live = MODE != REG_ROWS || x0 + l < kp.na;
+                    const bool live = !reg_strided(MODE) || x0 + l < kp.na;
                     if (ph == 0) PH::sweep(kp, sm, h, l, s);
                     else if (ph == 1) PH::link(kp, sm, h, l, s);
                     else if (ph == 2) PH::close(kp, sm, h, l, s);
                     else PH::out(kp, sm, h, l, s, kp.out + (live ? x0 + l + p * kp.pstride : 0), live);
                 }
-        if (MODE != REG_ROWS)
+        if (!reg_strided(MODE))
             for (int l = 0; l < LT && x0 + l < lim; ++l)
                 for (int r = 0; r < kp.n; ++r) {
                     double *d = kp.out + (x0 + l) * kp.n + r;

@@ -23,6 +23,10 @@ RegFn pick(int mode, int lines)
         if (lines == 32) return reg_kernel<RK, PER, M, EVEN, REG_ROWS, 32>;
         return lines == 16 ? reg_kernel<RK, PER, M, EVEN, REG_ROWS, 16> : reg_kernel<RK, PER, M, EVEN, REG_ROWS, 8>;
     }
+    if (mode == REG_ODD) {
+        if (lines == 32) return reg_kernel<RK, PER, M, EVEN, REG_ODD, 32>;
+        return lines == 16 ? reg_kernel<RK, PER, M, EVEN, REG_ODD, 16> : reg_kernel<RK, PER, M, EVEN, REG_ODD, 8>;
+    }
     if constexpr (reg_stagg(RK)) return nullptr;
     else if (mode == REG_SWZ)
         return lines == 16 ? reg_kernel<RK, PER, M, EVEN, REG_SWZ, 16> : reg_kernel<RK, PER, M, EVEN, REG_SWZ, 8>;

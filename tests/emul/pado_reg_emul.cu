@@ -15,7 +15,8 @@ constexpr int LT = 8;
 template <int RK, bool PER, int M, bool EVEN>
 int run_mode(const RegParams &kp, int mode)
 {
-    if (mode == REG_ROWS || reg_stagg(RK)) emulate_reg<RK, PER, M, EVEN, REG_ROWS, LT>(kp);
+    if (mode == REG_ODD) emulate_reg<RK, PER, M, EVEN, REG_ODD, LT>(kp);
+    else if (mode == REG_ROWS || reg_stagg(RK)) emulate_reg<RK, PER, M, EVEN, REG_ROWS, LT>(kp);
     else if constexpr (!reg_stagg(RK)) {
         if (mode == REG_SWZ) emulate_reg<RK, PER, M, EVEN, REG_SWZ, LT>(kp);
         else emulate_reg<RK, PER, M, EVEN, REG_PACK, LT>(kp);
@@ -64,13 +65,14 @@ extern "C" int emul_reg(int scheme, int kind, int n, double dx, int periodic, in
     kp.out_alpha = alpha;
     kp.nlines = (long long)na * nb;
     kp.stages = 1;
-    if (mode == REG_ROWS) {
+    if (reg_strided(mode)) {
+        kp.odd_rows = (n + 2) / 2 * (LT + 2);
         kp.na = (int)na;
         kp.xblocks = (int)((na + LT - 1) / LT);
         kp.ntiles = (long long)kp.xblocks * nb;
         kp.stride = axis == 2 ? na : na * (long long)nb;
         kp.pstride = axis == 2 ? na * (long long)n : na;
-        kp.tile_doubles = n * LT;
+        kp.tile_doubles = mode == REG_ODD ? (2 * kp.odd_rows + 15) / 16 * 16 : n * LT;
     } else {
         kp.ntiles = (kp.nlines + LT - 1) / LT;
         kp.P = n | 1;
@@ -88,7 +90,7 @@ extern "C" int emul_reg(int scheme, int kind, int n, double dx, int periodic, in
 // One operator of the staggered scheme on (n1, nin) lines along z; par: alpha,
 // a, b, sign; lhs: lower, diagonal and upper rows; rows: closure rows.
 extern "C" int emul_reg_stagg(int rk, int n, int nin, int periodic, int copy_first, const double *par, const double *lhs,
-                              const double *rows, int m, const double *f, double *df, long n1)
+                              const double *rows, int m, int mode, const double *f, double *df, long n1)
 {
     if (n < REG_MIN_N) return -3;
     RegCut cut;
@@ -120,11 +122,12 @@ extern "C" int emul_reg_stagg(int rk, int n, int nin, int periodic, int copy_fir
     kp.xblocks = (int)((n1 + LT - 1) / LT);
     kp.ntiles = kp.xblocks;
     kp.pstride = n1;
-    kp.tile_doubles = (nin + 15) / 16 * 16 * LT;
+    kp.odd_rows = (nin + 2) / 2 * (LT + 2);
+    kp.tile_doubles = (2 * kp.odd_rows + 15) / 16 * 16;
     switch (rk) {
-    case RHS_ST_EC: return run_rk<RHS_ST_EC>(kp, st.periodic, cut.even(), m, REG_ROWS);
-    case RHS_ST_CE: return run_rk<RHS_ST_CE>(kp, st.periodic, cut.even(), m, REG_ROWS);
-    case RHS_ST_D1: return run_rk<RHS_ST_D1>(kp, st.periodic, cut.even(), m, REG_ROWS);
-    default: return run_rk<RHS_ST_D2>(kp, st.periodic, cut.even(), m, REG_ROWS);
+    case RHS_ST_EC: return run_rk<RHS_ST_EC>(kp, st.periodic, cut.even(), m, mode);
+    case RHS_ST_CE: return run_rk<RHS_ST_CE>(kp, st.periodic, cut.even(), m, mode);
+    case RHS_ST_D1: return run_rk<RHS_ST_D1>(kp, st.periodic, cut.even(), m, mode);
+    default: return run_rk<RHS_ST_D2>(kp, st.periodic, cut.even(), m, mode);
     }
 }

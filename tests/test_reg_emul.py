@@ -5,6 +5,7 @@ segment length and tile layout, line lengths at the edges of the cuts (one
 segment, none, the most shared rows), closures, output modes.  Bar: 1e-12 of
 max |oracle|, as everywhere."""
 import ctypes
+import itertools
 
 import numpy as np
 import pytest
@@ -12,7 +13,7 @@ import pytest
 import oracle
 
 OPS = [(oracle.CD06, oracle.D1), (oracle.CD10, oracle.D1), (oracle.CD10, oracle.D2), (oracle.CF90, oracle.FILTER)]
-ROWS, SWZ, PACK = 0, 1, 2
+ROWS, SWZ, PACK, ODD = 0, 1, 2, 3
 
 
 @pytest.fixture(scope="module")
@@ -22,7 +23,7 @@ def emul():
     lib = ctypes.CDLL(build())
     P, I, D, Lg = ctypes.c_void_p, ctypes.c_int, ctypes.c_double, ctypes.c_long
     lib.emul_reg.argtypes = [I, I, I, D, I, I, I, I, I, I, I, I, I, D, P, P, Lg, Lg]
-    lib.emul_reg_stagg.argtypes = [I, I, I, I, I, P, P, P, I, P, P, Lg]
+    lib.emul_reg_stagg.argtypes = [I, I, I, I, I, P, P, P, I, I, P, P, Lg]
     return lib
 
 
@@ -43,7 +44,7 @@ def test_register_kernel_emulated(emul, scheme, kind, periodic):
         bcs = [(0, 0)] if periodic or scheme == oracle.CD06 else [(0, 0), (1, -1), (-1, 1)]
         for bc in bcs:
             op = oracle.OracleOp(scheme, n, dx, periodic, *bc)
-            for axis, mode in ((1, SWZ), (1, PACK), (2, ROWS), (3, ROWS)):
+            for axis, mode in ((1, SWZ), (1, PACK), (2, ROWS), (3, ROWS), (2, ODD), (3, ODD)):
                 f = rng.standard_normal({1: (3, 5, n), 2: (2, n, 11), 3: (n, 2, 11)}[axis])
                 na, nb = [s for a, s in enumerate(f.shape[::-1]) if a != axis - 1]
                 ref = op.apply(kind, axis, f, na, nb, *bc).reshape(f.shape)
@@ -136,14 +137,14 @@ def test_staggered_operators_emulated(emul, name, n):
         par = np.array([alpha, a / dx ** order, b / dx ** order, sign])
         lhs = np.ascontiguousarray(lhs)
         ran = 0
-        for m in (8, 16, 32):
+        for m, mode in itertools.product((8, 16, 32), (ROWS, ODD)):
             out = np.full_like(ref, np.nan)
             rc = emul.emul_reg_stagg(rk, solved, nin, int(setup[0]), int(setup[0] and nout > n), par.ctypes.data,
-                                     lhs.ctypes.data, rows.ctypes.data, m, f.ctypes.data, out.ctypes.data, 13)
+                                     lhs.ctypes.data, rows.ctypes.data, m, mode, f.ctypes.data, out.ctypes.data, 13)
             if rc == -2:
                 continue
             assert rc == 0
             ran += 1
             err = np.abs(out - ref).max() / np.abs(ref).max()
-            assert err <= 1e-12, (name, n, setup, m, err)
+            assert err <= 1e-12, (name, n, setup, m, mode, err)
         assert ran
