@@ -571,11 +571,14 @@ bool plan_reg(int rk, bool per, const RegCut &cut, long long na, long long nb, R
     // 16 lines 4790, 32 lines 4140).  x lines: 8, with a second buffer the
     // copies fill meanwhile (cd10 d1, n = 512 bounded: 5640 against 5030 with
     // 16 lines); 16 for short lines, which give 8 lines too few threads (n =
-    // 64 bounded: 4490 against 3490).
+    // 64 bounded: 4490 against 3490; cd10 d1 on 256^3 bounded 46 against 52 us).
     int L = S * 32 <= 512 ? 32 : (S * 16 <= 512 ? 16 : 8);
     if (rk == RHS_CF90 && L * S > 256 && L > 16) L = 16;
     if (xl && L > 16) L = 16;
-    if (mode == REG_SWZ && n > 128) L = 8;
+    if (mode == REG_SWZ && n > (per ? 128 : 256)) L = 8;
+    // a field of 64 MB stays in L2: more, smaller tiles there (cd06 on 128^3 6.0
+    // -> 5.4 us, cd10 d1 on 192^3 19.7 -> 18.2 us)
+    if (!xl && per && L > 16 && kp.nlines * n <= (8 << 20)) L = 16;
     // A strided tile's lines beyond the plane's edge are swept for nothing:
     // fewer lines per tile where that fills 15% more of them (cd10 d1 along y,
     // planes 33 wide: 2490 GB/s with 32 lines, 3550 with 8).

@@ -952,20 +952,19 @@ __global__ void __launch_bounds__(RegBounds<M>::threads, RegBounds<M>::ctas) reg
     const bool async = (MODE == REG_ROWS || MODE == REG_PACK) && kp.async_copy;
     const long long G = gridDim.x;
 
+    // the first copies start before the edge tables are staged
     if (tid == 0) {
         for (int b = 0; b < stages; ++b) mbar_init(&bars[b], async ? (unsigned)nthreads : 1u);
         mbar_fence_init();
+        if (!async)
+            for (int b = 0; b < stages; ++b)
+                if (blockIdx.x + b * G < kp.ntiles)
+                    reg_load<MODE, LT>(kp, base + (size_t)b * kp.tile_doubles, &bars[b], blockIdx.x + b * G);
     }
     if constexpr (!PER)
         for (int i = tid; i < edge_table; i += nthreads) base[lay.segtab + i] = __ldg(kp.segtab + i);
     __syncthreads();
-    if (async) {
-        if (blockIdx.x < kp.ntiles) reg_load_async<MODE, LT>(kp, base, &bars[0], blockIdx.x, tid, nthreads);
-    } else if (tid == 0) {
-        for (int b = 0; b < stages; ++b)
-            if (blockIdx.x + b * G < kp.ntiles)
-                reg_load<MODE, LT>(kp, base + (size_t)b * kp.tile_doubles, &bars[b], blockIdx.x + b * G);
-    }
+    if (async && blockIdx.x < kp.ntiles) reg_load_async<MODE, LT>(kp, base, &bars[0], blockIdx.x, tid, nthreads);
 
     const bool acc = kp.out_mode == OUT_ACC;
     if (acc && blockIdx.x < kp.ntiles) reg_prefetch<MODE, LT>(kp, blockIdx.x, tid, nthreads);
