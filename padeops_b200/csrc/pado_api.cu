@@ -109,7 +109,8 @@ void build_reg(pado_op_s *op, const std::vector<int> &kinds, const std::vector<s
         // the longer link and close steps (GB/s along x / y / z, 32 -> 16 rows:
         // n = 128 5539 / 5257 / 5195 -> 5905 / 6056 / 5911; n = 64 5466 / 5293 /
         // 5237 -> 5269 / 5409 / 5332; bounded ones lose 10-25%)
-        const bool short_segments = op->scheme == CF90 && op->periodic && n <= 256;
+        // (lines that 16 does not divide keep 32: n = 255 along y 3380 against 4880)
+        const bool short_segments = op->scheme == CF90 && op->periodic && n <= 256 && n % 16 == 0;
         if (!choose_reg_cut(reg_rows(n, op->periodic != 0), even_starts, short_segments, &r->cut)) return;
         std::memset(&r->kp, 0, sizeof(r->kp));
         std::vector<double> tab;

@@ -10,7 +10,7 @@
 //
 // on cyclic lines exactly (a cyclic band is the product of its cyclic
 // factors), on bounded lines for the rows [EDGE, n - EDGE).  A line is cut
-// into S segments of M rows (neighbours overlap by 0 to MAX_OVERLAP rows when
+// into S segments of M rows (neighbours overlap by a few rows when
 // S M exceeds the rows to cover); thread (l, s) holds the M rows of segment s
 // of line l in registers and never writes them to memory before the result:
 //
@@ -60,7 +60,10 @@ namespace pado {
 constexpr int REG_MAXM = 32;      // longest segment
 constexpr int REG_MAXS = 64;      // most segments per line
 constexpr int REG_EDGE = 4;       // closure rows solved as a block at each end
-constexpr int REG_OVERLAP = 4;    // most rows two neighbouring segments share
+// Most rows two neighbouring segments of M share: with 8 of 32 every line of
+// 104 points or more cuts into 32s (cd06 of 99 rows 5100 -> 5660 GB/s along y,
+// cd10 d2 of 64 rows with walls 4820 -> 5780; with 4 such lines took 16s).
+PADO_HD constexpr int reg_overlap(int M) { return M >= 32 ? 8 : 4; }
 constexpr int REG_SEGTAB = 12;    // doubles per segment of the edge tables
 // Closure rows of the staggered scheme, as its right-hand sides group them:
 // up to 3 groups coef * (sum of mul * the 8 input rows next to the wall)
@@ -183,7 +186,7 @@ struct OddAt {
     const double *p[2], *lo[2], *hi[2];  // rows of even and odd k
     PADO_HD PADO_INLINE static const double *place(const double *const (&par)[2], int r)
     {
-        return par[r & 1] + (r >> 1) * RS;  // r may be negative: floor
+        return (r & 1 ? par[1] : par[0]) + (r >> 1) * RS;  // r may be negative: floor
     }
     PADO_HD PADO_INLINE OddAt(const double *const (&par)[2], int n, int start, int m, bool cyclic)
     {
@@ -198,8 +201,8 @@ struct OddAt {
     template <int M>
     PADO_HD PADO_INLINE double get(int k) const
     {
-        const double *const(&b)[2] = k < LOW ? lo : (k < M + HIGH ? p : hi);
-        return b[k & 1][(k >> 1) * RS];
+        if (k & 1) return (k < LOW ? lo[1] : (k < M + HIGH ? p[1] : hi[1]))[(k >> 1) * RS];
+        return (k < LOW ? lo[0] : (k < M + HIGH ? p[0] : hi[0]))[(k >> 1) * RS];
     }
 };
 
@@ -241,7 +244,7 @@ struct SwzAt {
 template <int M>
 struct RegThread {
     double x[M];
-    double2 yc, xc;  // states handed on and back
+    double2 xc;  // state handed back
     double2 P, Q;
 };
 
@@ -286,35 +289,35 @@ struct RegLine {
 
     // Stencil and both recurrences with zero incoming states.  f: rows -H ..
     // M + H - 1 of the segment; od, op: rows shared with the next and the
-    // previous segment.  again(i): f at row i once more (DIFF).
+    // previous segment.  again(i): f at row i once more (DIFF).  ys, xs: where
+    // the states the neighbours start from go, taken on the way (a store under
+    // a predicate is two instructions a row; held in registers they are five).
     template <class Load, class Again>
     PADO_HD PADO_INLINE static void sweep(const RegParams &kp, Th &t, int od, int op, const Load &load,
-                                          const Again &again, double2 &last)
+                                          const Again &again, double2 *ys, double2 *xs, double2 &last)
     {
+        constexpr int OV = reg_overlap(M);
         double win[9];
 #pragma unroll
         for (int k = 0; k < 9; ++k) win[k] = 0.0;
         double f[M + 2 * H];
         load(f);
-        double y1 = 0.0, y2 = 0.0;
-        t.yc.x = t.yc.y = 0.0;
+        double2 y;
+        y.x = y.y = 0.0;
 #pragma unroll
         for (int i = 0; i < M; ++i) {
 #pragma unroll
             for (int o = -H; o <= H; ++o) win[4 + o] = f[i + H + o];
-            double y = rhs_interior_fma(RK, PER, kp.taps, win);
-            if (!TRI && i > 1) y = fma(kp.np2, y2, y);
-            if (i > 0) y = fma(kp.np1, y1, y);
-            t.x[i] = y;
-            y2 = y1;
-            y1 = y;
-            if (EVEN ? i == M - 1 : (i >= M - 1 - REG_OVERLAP && i == M - 1 - od)) {
-                t.yc.x = y1;
-                t.yc.y = y2;
-            }
+            double r = rhs_interior_fma(RK, PER, kp.taps, win);
+            if (!TRI && i > 1) r = fma(kp.np2, y.y, r);
+            if (i > 0) r = fma(kp.np1, y.x, r);
+            t.x[i] = r;
+            y.y = y.x;
+            y.x = r;
+            if (EVEN ? i == M - 1 : (i >= M - 1 - OV && i == M - 1 - od)) *ys = y;
         }
-        double x1 = 0.0, x2 = 0.0;
-        t.xc.x = t.xc.y = 0.0;
+        double2 x;
+        x.x = x.y = 0.0;
 #pragma unroll
         for (int i = M - 1; i >= 0; --i) {
 #ifdef __CUDA_ARCH__
@@ -324,20 +327,15 @@ struct RegLine {
             if (DIFF && (i + 1) % 8 == 0) __syncwarp(__activemask());
 #endif
             double d = t.x[i];
-            if (!TRI && i < M - 2) d = fma(kp.np2, x2, d);
-            if (i < M - 1) d = fma(kp.np1, x1, d);
+            if (!TRI && i < M - 2) d = fma(kp.np2, x.y, d);
+            if (i < M - 1) d = fma(kp.np1, x.x, d);
             t.x[i] = DIFF ? d + again(i) : d;
-            x2 = x1;
-            x1 = d;
-            if (i == M - 2) {
-                last.x = d;
-                last.y = x2;
-            }
-            if (EVEN ? i == 0 : (i <= REG_OVERLAP && i == op)) {
-                t.xc.x = x1;
-                t.xc.y = x2;
-            }
+            x.y = x.x;
+            x.x = d;
+            if (i == M - 2) last = x;
+            if (!EVEN && i <= OV && i == op) *xs = x;
         }
+        if (EVEN) t.xc = x;
     }
 
     // Incoming y state of segment s, and its x state as the predecessor
@@ -362,6 +360,7 @@ struct RegLine {
             a = carry(kp.wrap, a, z);
         }
         t.P = a;
+        if (!EVEN) t.xc = sm.xs[s * L + l];
         const double *w = kp.w[EVEN ? 0 : op];
         if (TRI) {
             t.xc.x = fma(w[0], a.x, t.xc.x);
@@ -583,7 +582,7 @@ struct RegOut {
 #pragma unroll
             for (int i = 0; i < M; ++i) {
                 const double x = RL::corrected(kp, t, i, t.x[i]);
-                if (EVEN || i >= REG_OVERLAP || i >= op) dst[i * kp.stride] = x;
+                if (EVEN || i >= reg_overlap(M) || i >= op) dst[i * kp.stride] = x;
             }
             return;
         }
@@ -601,7 +600,7 @@ struct RegOut {
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 const double x = RL::corrected(kp, t, c + i, t.x[c + i]);
-                if (EVEN || c + i >= REG_OVERLAP || c + i >= op)
+                if (EVEN || c + i >= reg_overlap(M) || c + i >= op)
                     dst[(c + i) * kp.stride] = fma(kp.out_alpha, x, old[(c / 8) & 1][i]);
             }
         }
@@ -616,7 +615,7 @@ struct RegOut {
                 double2 x;
                 x.x = RL::corrected(kp, t, i, t.x[i]);
                 x.y = RL::corrected(kp, t, i + 1, t.x[i + 1]);
-                if (EVEN || i >= REG_OVERLAP || i >= op)
+                if (EVEN || i >= reg_overlap(M) || i >= op)
                     *reinterpret_cast<double2 *>(at.unit(i)) = x;
             }
         } else {
@@ -624,7 +623,7 @@ struct RegOut {
 #pragma unroll
             for (int i = 0; i < M; ++i) {
                 const double x = RL::corrected(kp, t, i, t.x[i]);
-                if (EVEN || i >= REG_OVERLAP || i >= op) p[i] = x;
+                if (EVEN || i >= reg_overlap(M) || i >= op) p[i] = x;
             }
         }
     }
@@ -682,7 +681,7 @@ struct RegPhases {
                 if (i & 1) pair = *reinterpret_cast<const double2 *>(at.unit(i - 1));
                 return i & 1 ? pair.y : pair.x;
             };
-            RL::sweep(kp, t, od, op, load, again, last);
+            RL::sweep(kp, t, od, op, load, again, sm.ys + (s * LT + l), sm.xs + (s * LT + l), last);
         } else if constexpr (MODE == REG_ODD) {
             const double *par[2];
             parities(kp, sm, l, par);
@@ -692,7 +691,7 @@ struct RegPhases {
                 for (int k = -H; k < M + H; ++k) f[k + H] = at.template get<M>(k);
             };
             auto again = [&](int i) { return at.template get<M>(i); };
-            RL::sweep(kp, t, od, op, load, again, last);
+            RL::sweep(kp, t, od, op, load, again, sm.ys + (s * LT + l), sm.xs + (s * LT + l), last);
         } else {
             constexpr int RS = MODE == REG_ROWS ? LT : 1;
             const RowsAt<RS, RK> at(MODE == REG_ROWS ? sm.tile + l : sm.tile + (long long)l * kp.P, kp.n, st, M, PER);
@@ -701,9 +700,8 @@ struct RegPhases {
                 for (int k = -H; k < M + H; ++k) f[k + H] = at.template get<M>(k);
             };
             auto again = [&](int i) { return at.template get<M>(i); };
-            RL::sweep(kp, t, od, op, load, again, last);
+            RL::sweep(kp, t, od, op, load, again, sm.ys + (s * LT + l), sm.xs + (s * LT + l), last);
         }
-        sm.ys[s * LT + l] = t.yc;
         if constexpr (!PER) {
             if (s == 0) {
                 double g[8];

@@ -195,7 +195,7 @@ bool reg_cut(int rows, int M, bool even_starts, RegCut *cut)
     cut->d0 = base * step;
     cut->nd1 = units % (S - 1);
     cut->d1 = cut->nd1 ? (base + 1) * step : cut->d0;
-    return std::max(cut->d0, cut->d1) <= REG_OVERLAP;
+    return std::max(cut->d0, cut->d1) <= reg_overlap(M);
 }
 
 namespace {

@@ -14,7 +14,7 @@ struct RegCut {
     bool even() const { return d0 == 0 && nd1 == 0; }
 };
 // The cut of `rows` rows into segments of M rows; false when the neighbours
-// would have to share more than REG_OVERLAP rows.  even_starts: every overlap
+// would have to share more than reg_overlap(M) rows.  even_starts: every overlap
 // even (x lines that move two rows at a time).
 bool reg_cut(int rows, int M, bool even_starts, RegCut *cut);
 

@@ -150,8 +150,8 @@ struct pado_stagg_s {
     int n = 0, periodic = 1, top_even = 1, bot_even = 1, top_sided = 0, bot_sided = 0, device = 0;
     double dx = 1.0;
     StaggOp ops[PADO_STAGG_NOPS];
-    double *d_tab = nullptr;  // edge tables of every operator
-    int *d_status = nullptr;  // bounded waits of the register kernel
+    unsigned char *d_tab = nullptr;  // every operator's tables
+    int *d_status = nullptr;         // bounded waits of the register kernel, in d_tab
 };
 
 namespace {
@@ -783,9 +783,9 @@ bool row_groups(const SRow &r, int first, double *out)
     return true;
 }
 
-// The register kernel's constants of an operator, edge tables appended to
-// `all` from *off; null when its line does not cut into segments.
-std::unique_ptr<RegOp> stagg_reg(const StaggOp &o, std::vector<double> *all, size_t *off)
+// The register kernel's constants of an operator and its edge tables; null
+// when its line does not cut into segments.
+std::unique_ptr<RegOp> stagg_reg(const StaggOp &o, std::vector<double> *tab)
 {
     if (o.nsolve < REG_MIN_N) return nullptr;
     auto r = std::make_unique<RegOp>();
@@ -807,63 +807,56 @@ std::unique_ptr<RegOp> stagg_reg(const StaggOp &o, std::vector<double> *all, siz
         if (!row_groups(o.rows[(size_t)row], i < REG_EDGE ? 0 : o.nin - 8, st.rows + i * REG_GROUPS * 9)) return nullptr;
     }
     std::memset(&r->kp, 0, sizeof(r->kp));
-    std::vector<double> tab;
-    reg_fill_stagg(st, r->cut, &r->kp, &tab);
-    *off = all->size();
-    all->insert(all->end(), tab.begin(), tab.end());
+    reg_fill_stagg(st, r->cut, &r->kp, tab);
     return r;
 }
 
 void free_ops(pado_stagg_s *h)
 {
     if (h->d_tab) cudaFree(h->d_tab);
-    if (h->d_status) cudaFree(h->d_status);
     h->d_tab = nullptr;
-    h->d_status = nullptr;
-    for (auto &o : h->ops) {
-        if (o.d_rows) cudaFree(o.d_rows);
-        if (o.d_fac) cudaFree(o.d_fac);
-        o.d_rows = nullptr;
-        o.d_fac = nullptr;
-    }
 }
 
+// Every operator's tables in one allocation and copy.
 int upload(pado_stagg_s *h)
 {
-    for (auto &o : h->ops) {
-        if (!o.valid) continue;
-        cudaError_t e = cudaMalloc(&o.d_rows, o.rows.size() * sizeof(SRow));
-        if (e == cudaSuccess) e = cudaMalloc(&o.d_fac, o.fac.size() * sizeof(double));
-        if (e == cudaSuccess)
-            e = cudaMemcpy(o.d_rows, o.rows.data(), o.rows.size() * sizeof(SRow), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess)
-            e = cudaMemcpy(o.d_fac, o.fac.data(), o.fac.size() * sizeof(double), cudaMemcpyHostToDevice);
-        if (e != cudaSuccess) {
-            free_ops(h);
-            return pado::cuda_fail(e);
-        }
-    }
-    std::vector<double> all;
-    size_t off[PADO_STAGG_NOPS] = {0};
+    std::vector<unsigned char> all;
+    auto put = [&](const void *p, size_t bytes) {
+        const size_t off = (all.size() + 255) / 256 * 256;
+        all.resize(off + bytes);
+        if (bytes) std::memcpy(all.data() + off, p, bytes);
+        return off;
+    };
+    size_t rows[PADO_STAGG_NOPS], fac[PADO_STAGG_NOPS], edge[PADO_STAGG_NOPS];
+    const size_t status = put(nullptr, 0);
+    all.resize(status + sizeof(int), 0);
     for (int k = 0; k < PADO_STAGG_NOPS; ++k) {
-        if (!h->ops[k].valid) continue;
-        interior(h, k, &h->ops[k]);
-        h->ops[k].reg = stagg_reg(h->ops[k], &all, &off[k]);
+        StaggOp &o = h->ops[k];
+        if (!o.valid) continue;
+        rows[k] = put(o.rows.data(), o.rows.size() * sizeof(SRow));
+        fac[k] = put(o.fac.data(), o.fac.size() * sizeof(double));
+        interior(h, k, &o);
+        std::vector<double> tab;
+        o.reg = stagg_reg(o, &tab);
+        edge[k] = put(tab.data(), tab.size() * sizeof(double));
     }
-    cudaError_t e = cudaMalloc(&h->d_status, sizeof(int));
-    if (e == cudaSuccess) e = cudaMemset(h->d_status, 0, sizeof(int));
-    if (e == cudaSuccess && !all.empty()) e = cudaMalloc(&h->d_tab, all.size() * sizeof(double));
-    if (e == cudaSuccess && !all.empty())
-        e = cudaMemcpy(h->d_tab, all.data(), all.size() * sizeof(double), cudaMemcpyHostToDevice);
+    cudaError_t e = cudaMalloc(&h->d_tab, all.size());
+    if (e == cudaSuccess) e = cudaMemcpy(h->d_tab, all.data(), all.size(), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         free_ops(h);
         return pado::cuda_fail(e);
     }
-    for (int k = 0; k < PADO_STAGG_NOPS; ++k)
-        if (RegOp *r = h->ops[k].reg.get()) {
-            r->kp.segtab = h->d_tab ? h->d_tab + off[k] : nullptr;
+    h->d_status = reinterpret_cast<int *>(h->d_tab + status);
+    for (int k = 0; k < PADO_STAGG_NOPS; ++k) {
+        StaggOp &o = h->ops[k];
+        if (!o.valid) continue;
+        o.d_rows = reinterpret_cast<SRow *>(h->d_tab + rows[k]);
+        o.d_fac = reinterpret_cast<double *>(h->d_tab + fac[k]);
+        if (RegOp *r = o.reg.get()) {
+            r->kp.segtab = reinterpret_cast<double *>(h->d_tab + edge[k]);
             r->kp.status = h->d_status;
         }
+    }
     return PADO_OK;
 }
 
