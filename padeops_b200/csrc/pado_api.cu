@@ -562,7 +562,9 @@ bool plan_reg(int rk, bool per, const RegCut &cut, long long na, long long nb, R
     const bool odd = !xl && na % 2 && (axis == 2 || nb == 1) && !(reinterpret_cast<size_t>(kp.in) & 15) &&
                      na * (nb * nin) <= 0x7fffffffLL;
     const bool span = xl && n % 2 && !(align_bits & 15);
-    const int mode = xl ? (tma_ok ? REG_SWZ : REG_PACK) : (odd ? REG_ODD : REG_ROWS);
+    // lines of more segments than a swizzled tile's kernel has threads for take per-element copies
+    const bool swz = tma_ok && 8 * S <= reg_max_threads(M, REG_SWZ);
+    const int mode = xl ? (swz ? REG_SWZ : REG_PACK) : (odd ? REG_ODD : REG_ROWS);
     const bool even = per && cut.even();
     // Lines per tile, measured on 2^25..2^26 points (GB/s).  Strided lines: as
     // many as 512 threads sweep (longer rows for the copy engine and DRAM:
@@ -590,7 +592,7 @@ bool plan_reg(int rk, bool per, const RegCut &cut, long long na, long long nb, R
     }
     int stages = mode == REG_SWZ || span ? 2 : 1;
     kp.async_copy = mode == REG_PACK && !span ? 1 : 0;
-    const int max_threads = M >= 32 ? 512 : 384;
+    const int max_threads = reg_max_threads(M, mode);
     while (L > 8 && L * S > max_threads) L /= 2;
     const int threads = (L * S + 31) / 32 * 32;
     if (threads > max_threads) return false;
@@ -624,7 +626,7 @@ bool plan_reg(int rk, bool per, const RegCut &cut, long long na, long long nb, R
     if (!grant_smem((const void *)out->fn)) return false;
     const int ctas = resident_ctas((const void *)out->fn, threads, out->smem);
     if (ctas < 1) return false;
-    if (tma_ok || odd) {
+    if (mode == REG_SWZ || mode == REG_ODD || (mode == REG_ROWS && tma_ok)) {
         EncodeTiledFn enc = encode_tiled();
         if (!enc) return false;
         auto map = [&](CUtensorMap *m, const double *p, int rank, const cuuint64_t *dims, const cuuint64_t *strides,

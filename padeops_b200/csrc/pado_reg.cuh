@@ -921,15 +921,15 @@ __device__ __forceinline__ void reg_prefetch(const RegParams &kp, long long t, i
 }
 
 // Registers: a segment of 32 rows takes 64 for its values and about 45 more,
-// so 512 threads fill an SM; shorter segments leave room for more threads.
-template <int M>
-struct RegBounds {
-    static constexpr int threads = M >= 32 ? 512 : 384;
-    static constexpr int ctas = M >= 32 ? 1 : 2;
-};
+// so 512 threads fill an SM; the swizzled x-line tiles, two buffers to a CTA,
+// leave room for 384 threads in shared memory anyway, and their kernels take
+// the registers (bounded cf90 along x, n = 512: 28 spilled with 128, 4680 ->
+// 5600 GB/s); shorter segments leave room for more threads.
+PADO_HD constexpr int reg_max_threads(int M, int mode) { return M >= 32 && mode != REG_SWZ ? 512 : 384; }
+PADO_HD constexpr int reg_min_ctas(int M) { return M >= 32 ? 1 : 2; }
 
 template <int RK, bool PER, int M, bool EVEN, int MODE, int LT>
-__global__ void __launch_bounds__(RegBounds<M>::threads, RegBounds<M>::ctas) reg_kernel(const __grid_constant__ RegParams kp)
+__global__ void __launch_bounds__(reg_max_threads(M, MODE), reg_min_ctas(M)) reg_kernel(const __grid_constant__ RegParams kp)
 {
     using PH = RegPhases<RK, PER, M, EVEN, MODE, LT>;
     using RO = RegOut<RK, PER, M, EVEN, MODE, LT>;
