@@ -640,15 +640,18 @@ struct RegOut {
     PADO_HD PADO_INLINE static void edge(const RegParams &kp, const RegSmem &sm, const double (&e)[REG_EDGE], int l,
                                          int row0, double *line, bool live)
     {
+        if constexpr (reg_strided(MODE)) {
+            if (!live) return;
+            // df's values first: one wait for the four of them
+            double old[REG_EDGE];
 #pragma unroll
-        for (int i = 0; i < REG_EDGE; ++i) {
-            if constexpr (reg_strided(MODE)) {
-                double *d = line + (row0 + i) * kp.stride;
-                if (live) *d = kp.out_mode == OUT_ACC ? fma(kp.out_alpha, e[i], *d)
-                                                      : (kp.out_mode == OUT_SCALE ? kp.out_alpha * e[i] : e[i]);
-            } else {
-                *at(kp, sm.tile, l, row0 + i) = e[i];
-            }
+            for (int i = 0; i < REG_EDGE; ++i) old[i] = kp.out_mode == OUT_ACC ? line[(row0 + i) * kp.stride] : 0.0;
+#pragma unroll
+            for (int i = 0; i < REG_EDGE; ++i)
+                line[(row0 + i) * kp.stride] = kp.out_mode == OUT_STORE ? e[i] : fma(kp.out_alpha, e[i], old[i]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < REG_EDGE; ++i) *at(kp, sm.tile, l, row0 + i) = e[i];
         }
     }
 };
