@@ -59,9 +59,9 @@ def measured_peaks() -> tuple[float, str]:
 
 
 def profiled_traffic() -> float | None:
-    """DRAM bytes per 512^3 launch of the streaming kernel from the committed ncu
-    summary (profiles/stream_kernel_512cube.md, line 'traffic_bytes_per_launch: X')."""
-    p = os.path.join(ROOT, "profiles", "stream_kernel_512cube.md")
+    """DRAM bytes per 512^3 launch of the register kernel from the committed ncu
+    summary (profiles/register_kernel_512cube.md, line 'traffic_bytes_per_launch: X')."""
+    p = os.path.join(ROOT, "profiles", "register_kernel_512cube.md")
     try:
         with open(p) as fh:
             for line in fh:
@@ -527,7 +527,7 @@ def run_gpu(args) -> None:
                 "config": dict(CONFIG, per_operator_gbs=per_op),
                 "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                              "frac": round(achieved / peak, 4), "traffic": profiled_traffic(),
-                             "kernel": "pado::stream_kernel (the 9 launches of a step, averaged)",
+                             "kernel": "pado::reg_kernel (the 9 launches of a step, averaged)",
                              "peak_source": peak_kind},
                 "cpu_baseline": cpu, "e2e": e2e, "clocks": clk.summary(), "gpu_launches": launches,
                 "extensions": ext}

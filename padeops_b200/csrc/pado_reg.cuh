@@ -37,14 +37,15 @@
 // 5e-6), so the near-singular A (condition number near 2000) amplifies the
 // rounding of d and not that of f; f is added when d is complete.
 //
-// What bounds it: HBM, at 84-91% of the measured copy rate (6448 GB/s) for the
-// derivatives and 64-95% for cf90.  Per point the kernel issues the stencil (5
+// What bounds it: HBM, at 90-95% of the measured copy rate (6448 GB/s) for the
+// derivatives and 81-95% for cf90.  Per point the kernel issues the stencil (5
 // to 10 FP64), 4 recurrence and 4 correction FMAs, 1 + 2 H / M shared loads (H
-// the stencil's half width) and one store, against 67 to 90 instructions of
-// the streaming kernel, which keeps the line in shared memory and passes over
-// it four times.  B200, 512^3, x + y + z, streaming kernel -> this kernel:
-// cd10 d1 1928 -> 1191 us, cd10 d2 1983 -> 1139 us, cf90 2319 -> 1287 us;
-// 1024x512x256 with walls in z: cd06 1663 -> 1133 us, cd10 d1 1991 -> 1131 us.
+// the stencil's half width) and one store -- 31 (cd10 d1) to 56 (bounded cf90)
+// instructions in all -- against 67 to 90 of the streaming kernel, which keeps
+// the line in shared memory and passes over it four times.  B200, 512^3, x + y
+// + z, streaming kernel -> this kernel: cd10 d1 1929 -> 1070 us, cd10 d2 1985
+// -> 1065 us, cf90 2319 -> 1111 us; 1024x512x256 with walls in z: cd06 1664 ->
+// 1096 us, cd10 d1 1999 -> 1079 us.
 #pragma once
 
 #include <cuda.h>
