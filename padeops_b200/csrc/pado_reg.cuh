@@ -817,7 +817,8 @@ __device__ __forceinline__ int reg_span(const RegParams &kp, long long x0)
     return (int)(left < LT ? left : LT) * kp.n;
 }
 
-// Tensor or bulk copies of tile t into `tile` (one thread).
+// Tensor or bulk copies of tile t into `tile` (one thread, that which stores
+// the results: what it writes itself is seen from the barrier before the sweep).
 template <int MODE, int LT>
 __device__ __forceinline__ void reg_load(const RegParams &kp, double *tile, unsigned long long *bar, long long t)
 {
@@ -838,10 +839,15 @@ __device__ __forceinline__ void reg_load(const RegParams &kp, double *tile, unsi
             tma_load_2d(dst + kp.odd_rows, &kp.tin2, bar, (int)x0, (r0 >> 1) + b * kp.box_rows);
         }
     } else if constexpr (MODE == REG_PACK) {
-        // whole 16-byte units of the span (tiles start on them: LT is even)
-        const unsigned bytes = ((unsigned)reg_span<LT>(kp, x0) * 8u) & ~15u;
+        // whole 16-byte units of the span (tiles start on them: LT is even), and
+        // the last element of a field of an odd number of them, by this thread
+        // as well: it alone has waited for the tile's last results to be read
+        const int total = reg_span<LT>(kp, x0);
+        const unsigned bytes = ((unsigned)total * 8u) & ~15u;
+        const double *src = kp.in + x0 * (long long)kp.n;
         mbar_expect_tx(bar, bytes);
-        bulk_load(tile, kp.in + x0 * (long long)kp.n, bytes, bar);
+        bulk_load(tile, src, bytes, bar);
+        if (total & 1) tile[total - 1] = __ldg(src + total - 1);
     } else {
         mbar_expect_tx(bar, (unsigned)kp.nbox * kp.box_rows * LT * 8u);
         for (int b = 0; b < kp.nbox; ++b) {
@@ -973,14 +979,6 @@ __global__ void __launch_bounds__(reg_max_threads(M, MODE), reg_min_ctas(M)) reg
     int b = 0;
     unsigned parity = 0;
     for (long long t = blockIdx.x; t < kp.ntiles; t += G) {
-        if (MODE == REG_PACK && !async && tid == nthreads - 1) {
-            // a last tile of an odd number of elements: the one past its whole units
-            long long x0, p;
-            reg_origin(kp, LT, t, &x0, &p);
-            const int total = reg_span<LT>(kp, x0);
-            if (total & 1)
-                base[(size_t)b * kp.tile_doubles + total - 1] = __ldg(kp.in + x0 * (long long)kp.n + total - 1);
-        }
         bool arrived = true;
         if (tid < 32) arrived = mbar_wait(&bars[b], parity, STREAM_WAIT_NS);
         if (!__syncthreads_and(arrived)) {

@@ -68,3 +68,39 @@ def test_register_kernel_long_lines(scheme, kind, n):
             assert op.device_status() == 0
             ref = _oracle_apply(scheme, kind, axis, f, 0.3, periodic, 0, 0)
             assert rel_err(out.cpu().numpy(), ref) <= TOL, (periodic, axis)
+
+
+@pytest.mark.parametrize("scheme,kind", OPS)
+@pytest.mark.parametrize("n,n2,n3", [(1023, 69, 35), (1701, 109, 11)])
+def test_register_kernel_odd_lines_one_buffer(scheme, kind, n, n2, n3):
+    """x lines of an odd length for which one tile buffer fits, a field of an odd number of elements (a last
+    tile of 15 or 7 lines) and more tiles than CTAs: a CTA places the field's last element in the buffer whose
+    results it has just handed to the copy engine.  Whole outputs, 50 times over."""
+    import torch
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    rng = np.random.default_rng(n + 3 * scheme + kind)
+    f = rng.standard_normal((n3, n2, n))
+    df0 = rng.standard_normal(f.shape)
+    ft, df0t = torch.from_numpy(f).cuda(), torch.from_numpy(df0).cuda()
+    for periodic in (True, False):
+        op = _make(scheme, n, 0.3, periodic)
+        out = torch.empty_like(ft)
+        plan = op.launch_plan(kind, 1, ft, out, n2, n3)
+        tiles = -(-n2 * n3 // plan["lines"])
+        assert plan["stages"] == 1 and tiles > plan["ctas_per_sm"] * sms, plan
+        assert n2 * n3 % plan["lines"] == plan["lines"] - 1
+        ref = _oracle_apply(scheme, kind, 1, f, 0.3, periodic, 0, 0)
+        for alpha, beta in ((1.0, 0.0), (-0.75, 1.0)):
+            first = None
+            for _ in range(50):
+                if beta:
+                    out.copy_(df0t)
+                else:
+                    out.fill_(float("nan"))
+                op.apply(kind, 1, ft, out, n2, n3, alpha=alpha, beta=beta)
+                if first is None:
+                    first = out.clone()
+                    assert rel_err(first.cpu().numpy(), alpha * ref + beta * df0) <= TOL, (periodic, beta)
+                assert torch.equal(out, first), (periodic, beta)
+        assert op.device_status() == 0
