@@ -1150,13 +1150,13 @@ int pado_set_tiling(pado_op_t op, int m, int lines)
     const int om = op->m, ol = op->lines;
     if (m) op->m = m;
     if (lines) op->lines = lines;
-    op->tiled = m != 0 || lines != 0;
     const int S = (op->n + op->m - 1) / op->m;
     if (S > 32) {
         op->m = om;
         op->lines = ol;
         return PADO_E_SIZE;
     }
+    op->tiled = m != 0 || lines != 0;
     if (op->m != om) return build_tables(op);
     return PADO_OK;
 }

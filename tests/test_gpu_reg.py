@@ -104,3 +104,18 @@ def test_register_kernel_odd_lines_one_buffer(scheme, kind, n, n2, n3):
                     assert rel_err(first.cpu().numpy(), alpha * ref + beta * df0) <= TOL, (periodic, beta)
                 assert torch.equal(out, first), (periodic, beta)
         assert op.device_status() == 0
+
+
+@pytest.mark.parametrize("scheme,kind", OPS)
+def test_refused_tiling_changes_nothing(scheme, kind):
+    """Segments of 16 rows do not cover 1024: the call is refused, and the handle launches what it did."""
+    import torch
+
+    from padeops_b200 import PadoError
+
+    op = _make(scheme, 1024, 0.3, True)
+    ft = torch.zeros((4, 64, 1024), dtype=torch.float64, device="cuda")
+    before = op.launch_plan(kind, 1, ft, torch.empty_like(ft), 64, 4)
+    with pytest.raises(PadoError):
+        op.set_tiling(16, 8)
+    assert op.launch_plan(kind, 1, ft, torch.empty_like(ft), 64, 4) == before
