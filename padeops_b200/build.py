@@ -20,7 +20,8 @@ LIB = os.path.join(LIBDIR, "libpado.so")
 SOURCES = ["pado_api.cu", "pado_batch.cu", "pado_tables.cpp", "pado_inst.cu", "pado_stagg.cu",
            "pado_reg_inst.cu", "pado_reg_tables.cpp"]
 HEADERS = ["pado_common.h", "pado_tables.h", "pado_kernels.cuh", "pado_batch.cuh", "pado_internal.h", "pado_params.h",
-           "pado_stream.cuh", "pado_resident.cuh", "pado_reg.cuh", "pado_reg_tables.h"]
+           "pado_stream.cuh", "pado_resident.cuh", "pado_reg.cuh", "pado_reg_tables.h",
+           "pado_once.h"]
 # pado_inst.cu is compiled once per stencil (-DPADO_RK=n) into pado_inst_rkN.o
 STENCILS = 4
 # pado_reg_inst.cu once per stencil and segment length (-DPADO_RM=m) into pado_reg_inst_rkN_m.o

@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "pado_internal.h"
+#include "pado_once.h"
 
 #include <algorithm>
 
@@ -236,22 +237,22 @@ int stream_tile_doubles(bool xl, int n, int L, bool as)
     return round16((long long)nbox * box_rows * L);
 }
 
-// Lets a streaming kernel use up to 227 KB of shared memory (once per kernel).
+int current_device()
+{
+    int dev = 0;
+    cudaGetDevice(&dev);
+    return dev;
+}
+
+// Lets a kernel use up to 227 KB of shared memory (once per kernel and device).
 bool grant_smem(const void *fn)
 {
-    static std::mutex mu;
-    static std::map<const void *, bool> granted;
-    std::lock_guard<std::mutex> g(mu);
-    bool &ok = granted[fn];
-    if (!ok) {
-        if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) !=
-            cudaSuccess) {
-            (void)cudaGetLastError();
-            return false;
-        }
-        ok = true;
-    }
-    return true;
+    static OncePerDevice<const void *, bool> granted;
+    return granted.get(fn, current_device(), [&] {
+        const bool ok = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) == cudaSuccess;
+        if (!ok) (void)cudaGetLastError();
+        return ok;
+    });
 }
 
 // Plan of a streaming launch (primal): lines per tile, stages, shared memory
@@ -468,8 +469,8 @@ int sm_count()
 {
     constexpr int MAX_DEVICES = 64;
     static std::atomic<int> known[MAX_DEVICES];
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
+    int sms = 0;
+    const int dev = current_device();
     if (dev >= 0 && dev < MAX_DEVICES && (sms = known[dev].load(std::memory_order_relaxed)) > 0) return sms;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (sms < 1) return 1;
@@ -528,20 +529,13 @@ RegFn pick_reg(int rk, int m, bool per, bool even, int mode, int lines)
 // asked of the runtime once per shape and device.
 int resident_ctas(const void *fn, int threads, size_t smem)
 {
-    static std::mutex mu;
-    static std::map<std::tuple<const void *, int, size_t, int>, int> known;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    const std::tuple<const void *, int, size_t, int> key(fn, threads, smem, dev);
-    std::lock_guard<std::mutex> g(mu);
-    const auto it = known.find(key);
-    if (it != known.end()) return it->second;
-    int ctas = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, fn, threads, smem) != cudaSuccess) {
+    static OncePerDevice<std::tuple<const void *, int, size_t>, int> known;
+    return known.get({fn, threads, smem}, current_device(), [&] {
+        int ctas = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, fn, threads, smem) == cudaSuccess) return ctas;
         (void)cudaGetLastError();
         return 0;
-    }
-    return known[key] = ctas;
+    });
 }
 
 bool plan_reg(int rk, bool per, const RegCut &cut, long long na, long long nb, RegLaunch *out)

@@ -8,7 +8,7 @@ OUT = os.path.join(HERE, "_build", "libpado_reg_emul.so")
 SRCS = [os.path.join(HERE, "pado_reg_emul.cu")] + [os.path.join(CSRC, f) for f in ("pado_reg_tables.cpp",
                                                                                    "pado_tables.cpp")]
 DEPS = SRCS + [os.path.join(CSRC, h) for h in ("pado_reg.cuh", "pado_reg_tables.h", "pado_common.h", "pado_kernels.cuh",
-                                               "pado_stream.cuh", "pado_resident.cuh", "pado_tables.h")]
+                                               "pado_stream.cuh", "pado_resident.cuh", "pado_tables.h", "pado_once.h")]
 
 
 def build() -> str:

@@ -4,6 +4,7 @@
 #include <cstring>
 #include <vector>
 
+#include "../../padeops_b200/csrc/pado_once.h"
 #include "../../padeops_b200/csrc/pado_reg_tables.h"
 
 using namespace pado;
@@ -129,5 +130,19 @@ extern "C" int emul_reg_stagg(int rk, int n, int nin, int periodic, int copy_fir
     case RHS_ST_CE: return run_rk<RHS_ST_CE>(kp, st.periodic, cut.even(), m, mode);
     case RHS_ST_D1: return run_rk<RHS_ST_D1>(kp, st.periodic, cut.even(), m, mode);
     default: return run_rk<RHS_ST_D2>(kp, st.periodic, cut.even(), m, mode);
+    }
+}
+
+// Calls of one kernel on device dev[i], whose runtime would answer answer[i]:
+// what each call got, and whether the runtime was asked.
+extern "C" void emul_once_per_device(int calls, const int *dev, const int *answer, int *got, int *asked)
+{
+    OncePerDevice<const void *, int> once;
+    for (int i = 0; i < calls; ++i) {
+        asked[i] = 0;
+        got[i] = once.get(nullptr, dev[i], [&] {
+            asked[i] = 1;
+            return answer[i];
+        });
     }
 }

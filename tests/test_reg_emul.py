@@ -148,3 +148,12 @@ def test_staggered_operators_emulated(emul, name, n):
             err = np.abs(out - ref).max() / np.abs(ref).max()
             assert err <= 1e-12, (name, n, setup, m, mode, err)
         assert ran
+
+
+def test_runtime_answers_are_kept_per_device(emul):
+    """A kernel's shared-memory grant and occupancy: asked once on each device, again after a failure (0)."""
+    V = ctypes.c_int * 6
+    got, asked = V(), V()
+    emul.emul_once_per_device(6, V(0, 0, 1, 1, 1, 0), V(3, 9, 0, 2, 9, 9), got, asked)
+    assert list(got) == [3, 3, 0, 2, 2, 3]
+    assert list(asked) == [1, 0, 1, 1, 0, 0]
