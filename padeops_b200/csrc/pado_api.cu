@@ -452,15 +452,13 @@ bool plan_reg_op(const pado_op_s *op, const RegOp &ro, int kind, int axis, const
 // The register kernel's constants for a request, or null when another kernel
 // runs it: an explicit kernel or tiling, a short or uncuttable line, the
 // adjoint of a bounded line.
-const RegOp *reg_op(const pado_op_s *op, int kind, int axis, const double *f, const double *df, int bc1, int bcn,
-                    bool adj, int solve_bc1, int solve_bcn)
+const RegOp *reg_op(const pado_op_s *op, int kind, int axis, int bc1, int bcn, bool adj, int solve_bc1, int solve_bcn)
 {
     if (op->variant != 0 || op->stream_lines || op->stream_stages || op->tiled || (adj && !op->periodic)) return nullptr;
     const bool bounded_bc = !op->periodic && op->scheme != CD06;
     const int b1 = bounded_bc ? bc1 : 0, bn = bounded_bc ? bcn : 0;
     const int s1 = bounded_bc && solve_bc1 != SAME_BC ? solve_bc1 : b1, sn = bounded_bc && solve_bcn != SAME_BC ? solve_bcn : bn;
-    const bool even = axis == 1 && op->n % 2 == 0 && !((reinterpret_cast<size_t>(f) | reinterpret_cast<size_t>(df)) & 15);
-    const auto it = op->reg.find(RegKey(kind, b1, bn, s1, sn, even ? 1 : 0));
+    const auto it = op->reg.find(RegKey(kind, b1, bn, s1, sn, reg_even_starts(axis, op->n) ? 1 : 0));
     return it == op->reg.end() ? nullptr : it->second.get();
 }
 
@@ -775,7 +773,7 @@ int launch(pado_op_s *op, int kind, int axis, const double *f, double *df, long 
         }
         return e == cudaSuccess ? PADO_OK : cuda_fail(e);
     }
-    if (const RegOp *ro = reg_op(op, kind, axis, f, df, bc1, bcn, adjoint, solve_bc1, solve_bcn)) {
+    if (const RegOp *ro = reg_op(op, kind, axis, bc1, bcn, adjoint, solve_bc1, solve_bcn)) {
         RegLaunch r;
         if (plan_reg_op(op, *ro, kind, axis, f, df, na, nb, adjoint, out_mode, out_alpha, &r)) return launch_reg(r, st);
     }
@@ -1172,7 +1170,7 @@ int pado_launch_plan(pado_op_t op, int kind, int axis, const double *f, double *
     bool trivial = true;
     int rc = prepare_launch(op, kind, axis, f, df, na, nb, bc1, bcn, false, op ? op->lines : 0, false, &kp, &trivial);
     if (rc != PADO_OK || trivial) return rc;
-    if (const RegOp *ro = reg_op(op, kind, axis, f, df, bc1, bcn, false, SAME_BC, SAME_BC)) {
+    if (const RegOp *ro = reg_op(op, kind, axis, bc1, bcn, false, SAME_BC, SAME_BC)) {
         RegLaunch r;
         if (plan_reg_op(op, *ro, kind, axis, f, df, na, nb, false, OUT_STORE, 1.0, &r)) {
             const bool copies = r.mode == REG_PACK || r.mode == REG_ODD || r.kp.async_copy;

@@ -15,8 +15,14 @@ struct RegCut {
 };
 // The cut of `rows` rows into segments of M rows; false when the neighbours
 // would have to share more than reg_overlap(M) rows.  even_starts: every overlap
-// even (x lines that move two rows at a time).
+// even.
 bool reg_cut(int rows, int M, bool even_starts, RegCut *cut);
+
+// x lines of even length: the swizzled tile moves two rows at a time.  The
+// other copies of such a line (fields 8 bytes off a 16-byte boundary) take the
+// same cut, so that a result's rounding does not depend on where its field
+// lies; M and S are the same with any starts.
+inline bool reg_even_starts(int axis, int n) { return axis == 1 && n % 2 == 0; }
 
 // Rows of a line the segments cover.
 inline int reg_rows(int n, bool periodic) { return periodic ? n : n - 2 * REG_EDGE; }

@@ -53,7 +53,7 @@ extern "C" int emul_reg(int scheme, int kind, int n, double dx, int periodic, in
 {
     if (n < REG_MIN_N) return -3;
     RegCut cut;
-    if (!reg_cut(reg_rows(n, periodic != 0), m, mode == REG_SWZ, &cut)) return -2;
+    if (!reg_cut(reg_rows(n, periodic != 0), m, reg_even_starts(axis, n), &cut)) return -2;
     RegParams kp;
     std::memset(&kp, 0, sizeof(kp));
     std::vector<double> segtab;

@@ -119,3 +119,29 @@ def test_refused_tiling_changes_nothing(scheme, kind):
     with pytest.raises(PadoError):
         op.set_tiling(16, 8)
     assert op.launch_plan(kind, 1, ft, torch.empty_like(ft), 64, 4) == before
+
+
+@pytest.mark.parametrize("scheme,kind", OPS)
+def test_rounding_does_not_depend_on_the_address(scheme, kind):
+    """A field 8 bytes past a 16-byte boundary, input, output or both: other copies, the same bits."""
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(5 + scheme + kind)
+    for n in (50, 64, 90, 129, 200, 512, 1000):
+        for periodic in (True, False):
+            op = _make(scheme, n, 0.3, periodic)
+            for axis, cross in ((1, 22), (2, 22), (2, 21), (3, 22), (3, 21)):
+                shape = {1: (9, 11, n), 2: (9, n, cross), 3: (n, 9, cross)}[axis]
+                na, nb = na_nb(shape, axis)
+                size = n * na * nb
+                base = torch.randn(size, dtype=torch.float64, device="cuda", generator=g)
+                outs = []
+                for off_in, off_out in ((0, 0), (1, 0), (0, 1), (1, 1)):
+                    f = torch.zeros(size + 1, dtype=torch.float64, device="cuda")[off_in:off_in + size]
+                    f.copy_(base)
+                    out = torch.full((size + 1,), float("nan"), dtype=torch.float64, device="cuda")[off_out:off_out + size]
+                    op.apply(kind, axis, f, out, na, nb)
+                    outs.append(out)
+                for out in outs[1:]:
+                    assert torch.equal(out, outs[0]), (n, periodic, axis, cross)
+            assert op.device_status() == 0

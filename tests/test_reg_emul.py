@@ -62,6 +62,20 @@ def test_register_kernel_emulated(emul, scheme, kind, periodic):
     assert cuts > 60
 
 
+@pytest.mark.parametrize("scheme,kind", OPS)
+def test_x_lines_round_alike_in_every_tile(emul, scheme, kind):
+    """Even lengths whose cut shares rows: the swizzled and the packed tile give the same bits."""
+    rng = np.random.default_rng(8 + scheme + kind)
+    for n, m, periodic in itertools.product((50, 90, 200, 512, 1000), (8, 16, 32), (True, False)):
+        f = rng.standard_normal((3, 5, n))
+        outs = [np.full_like(f, np.nan) for _ in range(2)]
+        rcs = [_run(emul, scheme, kind, n, 0.3, periodic, (0, 0), (0, 0), m, mode, 1, 0, 1.0, f, out)
+               for mode, out in zip((SWZ, PACK), outs)]
+        assert rcs[0] == rcs[1]
+        if rcs[0] == 0:
+            assert np.array_equal(*outs), (n, m, periodic)
+
+
 def test_register_kernel_output_modes_emulated(emul):
     rng = np.random.default_rng(5)
     n = 72
