@@ -117,7 +117,9 @@ struct alignas(64) RegParams {
     double dtaps[2][REG_EDGE][8];  // cf90: rows of B - A on the 8 rows next to the wall
     double fr[2][2][REG_EDGE], fx[2][2][2];  // end state = fr r + fx (the two interior rows next to the block)
     double kinv[4][4];          // both ends together: (1 - K)^-1
-    double xr[2][REG_EDGE][REG_EDGE], xx[2][REG_EDGE][2];  // closure rows' x = xr r + xx (the two interior rows)
+    // closure rows, eliminated from the wall: x = xr r (its row's and those nearer the wall) + xx (the next two x inwards);
+    // cf90's, solved: x = xr r + xx (the two interior rows)
+    double xr[2][REG_EDGE][REG_EDGE], xx[2][REG_EDGE][2];
 };
 static_assert(sizeof(RegParams) <= 4096, "launch parameters");
 
@@ -523,19 +525,45 @@ struct RegLine {
         t.Q.x = fma(g[4], z[0], fma(g[5], z[1], fma(g[8], z[2], fma(g[9], z[3], t.Q.x))));
         t.Q.y = fma(g[6], z[0], fma(g[7], z[1], fma(g[10], z[2], fma(g[11], z[3], t.Q.y))));
     }
-    // x of the closure rows of one end, from the two interior rows next to it.
+    // x of the closure rows of one end, from the two interior rows next to it:
+    // substitution towards the wall.  (As a product with the block's inverse,
+    // every row of it from all four right-hand sides, the wall row's error was
+    // up to 1.4 times an elimination's: it takes its neighbours' with weights
+    // of 3 and 11.)  The filter's rows are that product: what it solves for is
+    // small beside f, to which it is then added, and the chain of four rows
+    // spills 8 bytes there (1024 rows along y and z, 220 -> 227 us).
     template <int SIDE>
     PADO_HD PADO_INLINE static void edge_rows(const RegParams &kp, const RegSmem &sm, int L, int l, double2 x,
                                               double (&out)[REG_EDGE])
     {
         const double *r = edge_r(sm, L, l, SIDE);
+        if (DIFF) {
 #pragma unroll
-        for (int i = 0; i < REG_EDGE; ++i) {
+            for (int i = 0; i < REG_EDGE; ++i) {
+                double a = fma(kp.xx[SIDE][i][0], x.x, kp.xx[SIDE][i][1] * x.y);
+#pragma unroll
+                for (int j = 0; j < REG_EDGE; ++j) a = fma(kp.xr[SIDE][i][j], r[j * L], a);
+                out[i] = a + edge_f(sm, L, l, SIDE)[i * L];
+            }
+            return;
+        }
+#pragma unroll
+        for (int k = REG_EDGE - 1; k >= 0; --k) {  // k-th row from the wall
+            const int i = SIDE ? REG_EDGE - 1 - k : k;
             double a = fma(kp.xx[SIDE][i][0], x.x, kp.xx[SIDE][i][1] * x.y);
 #pragma unroll
-            for (int j = 0; j < REG_EDGE; ++j) a = fma(kp.xr[SIDE][i][j], r[j * L], a);
-            if (DIFF) a += edge_f(sm, L, l, SIDE)[i * L];
+            for (int j = 0; j <= k; ++j) {
+                const int c = SIDE ? REG_EDGE - 1 - j : j;
+                a = fma(kp.xr[SIDE][i][c], r[c * L], a);
+            }
             out[i] = a;
+            if (SIDE) {
+                x.x = x.y;
+                x.y = a;
+            } else {
+                x.y = x.x;
+                x.x = a;
+            }
         }
     }
     // The rows next to the blocks, complete.

@@ -201,8 +201,8 @@ bool reg_cut(int rows, int M, bool even_starts, RegCut *cut)
 namespace {
 
 // Everything that follows from the left-hand side alone: its band and, on
-// bounded lines, the closure rows A.
-void fill_system(const RegBand &rb, bool periodic, const ld (*A)[REG_EDGE][REG_EDGE + 2], const RegCut &cut,
+// bounded lines, the closure rows A; solved: how RegParams::xr holds them.
+void fill_system(const RegBand &rb, bool periodic, const ld (*A)[REG_EDGE][REG_EDGE + 2], bool solved, const RegCut &cut,
                  RegParams *kp, std::vector<double> *segtab)
 {
     const int M = cut.M, S = cut.S, n = rb.n;
@@ -256,21 +256,40 @@ void fill_system(const RegBand &rb, bool periodic, const ld (*A)[REG_EDGE][REG_E
 
     // ---- bounded: the closure blocks and the line between them --------------
     const int N = n - 2 * REG_EDGE;
-    // block rows: x = X r - X A2 (next two interior rows), X = A1^-1
+    // block rows, k-th from the wall: elimination inwards leaves each as its own
+    // right-hand side's and those before it and the two x further in; with these
+    // put in, all four right-hand sides and the two interior rows next to the block
     ld xr[2][REG_EDGE][REG_EDGE], xx[2][REG_EDGE][2];
     for (int side = 0; side < 2; ++side) {
-        ld m[REG_EDGE][REG_EDGE + REG_EDGE + 2];
-        for (int i = 0; i < REG_EDGE; ++i) {
-            for (int j = 0; j < REG_EDGE; ++j) {
-                m[i][j] = A[side][i][side ? j + 2 : j];
-                m[i][REG_EDGE + j] = i == j ? 1 : 0;
-            }
-            for (int k = 0; k < 2; ++k) m[i][2 * REG_EDGE + k] = -A[side][i][side ? k : REG_EDGE + k];
+        constexpr int E = REG_EDGE;
+        auto at = [&](int k, int end) { return side ? end - 1 - k : k; };
+        ld m[E][2 * E + 2], x[E][E + 2];
+        for (int i = 0; i < E; ++i) {
+            for (int j = 0; j < E + 2; ++j) m[i][j] = A[side][at(i, E)][at(j, E + 2)];
+            for (int j = 0; j < E; ++j) m[i][E + 2 + j] = i == j ? 1 : 0;
         }
-        solve<REG_EDGE, REG_EDGE + 2>(m);
-        for (int i = 0; i < REG_EDGE; ++i) {
-            for (int j = 0; j < REG_EDGE; ++j) kp->xr[side][i][j] = (double)(xr[side][i][j] = m[i][REG_EDGE + j]);
-            for (int k = 0; k < 2; ++k) kp->xx[side][i][k] = (double)(xx[side][i][k] = m[i][2 * REG_EDGE + k]);
+        for (int c = 0; c < E; ++c) {
+            const ld inv = 1 / m[c][c];
+            for (ld &v : m[c]) v *= inv;
+            for (int i = c + 1; i < E; ++i) {
+                const ld f = m[i][c];
+                for (int j = 0; j < 2 * E + 2; ++j) m[i][j] -= f * m[c][j];
+            }
+        }
+        for (int i = E - 1; i >= 0; --i)
+            for (int j = 0; j < E + 2; ++j) {
+                x[i][j] = j < E ? m[i][E + 2 + j] : (ld)0;
+                for (int k = i + 1; k <= i + 2; ++k) x[i][j] -= m[i][k] * (k < E ? x[k][j] : (ld)(k == j));
+            }
+        for (int i = 0; i < E; ++i) {
+            for (int j = 0; j < E; ++j) {
+                xr[side][at(i, E)][at(j, E)] = x[i][j];
+                kp->xr[side][at(i, E)][at(j, E)] = (double)(solved ? x[i][j] : m[i][E + 2 + j]);
+            }
+            for (int k = 0; k < 2; ++k) {
+                xx[side][at(i, E)][at(k, 2)] = x[i][E + k];
+                kp->xx[side][at(i, E)][at(k, 2)] = (double)(solved ? x[i][E + k] : -m[i][i + 1 + k]);
+            }
         }
     }
     // end states: left (y_3, y_2) with y_i = x_i + p1 x_{i+1} + p2 x_{i+2};
@@ -331,7 +350,7 @@ void reg_fill(const RegBand &rb, int scheme, int kind, double dx, bool periodic,
     const ld c = rb.c;
     ld A[2][REG_EDGE][REG_EDGE + 2];
     if (!periodic) edge_lhs(scheme, kind, sbc1, sbcn, A);
-    fill_system(rb, periodic, A, cut, kp, segtab);
+    fill_system(rb, periodic, A, scheme == CF90, cut, kp, segtab);
     kp->bc1 = bc1;
     kp->bcn = bcn;
     const RhsCoef rc = make_rhs_coef(scheme, kind, dx, periodic);
@@ -367,7 +386,7 @@ void reg_fill_stagg(const RegStagg &st, const RegCut &cut, RegParams *kp, std::v
         }
     const RegBand rb(n, st.periodic, st.alpha, 0);
     const ld c = rb.c;
-    fill_system(rb, st.periodic, A, cut, kp, segtab);
+    fill_system(rb, st.periodic, A, false, cut, kp, segtab);
     kp->nin = st.nin;
     kp->copy_first = st.copy_first;
     kp->taps[0] = (double)((ld)st.a / c);
