@@ -169,7 +169,7 @@ int pado_apply_host_terms(const double *f_host, long n1, long n2, long n3, const
 /* ---- tuning ------------------------------------------------------------- */
 
 /* Launch shape of the line kernels for this handle: m = segment length
- * (rows one thread solves serially, 8/16/32/64), lines = lines per CTA
+ * (rows one thread solves serially, 16/32/64), lines = lines per CTA
  * (8/16/32).  0 keeps the current value.  Rebuilds the handle's tables.
  * After a call that names m or lines the automatic choice keeps to the
  * kernels that take them; a call with two zeros gives it all of them back. */
@@ -204,17 +204,23 @@ int pado_set_kernel_variant(pado_op_t op, int variant);
  * reference (a B200 tuning knob). */
 int pado_set_stream_tiling(pado_op_t op, int lines, int stages);
 /* Device-side status of the handle's kernels: PADO_OK, or PADO_E_TIMEOUT
- * when a streaming kernel's bounded wait for its copies expired (its CTAs
+ * when a streaming or register kernel's bounded wait for its copies expired (its CTAs
  * then stop early and the output is incomplete).  Synchronous (reads device
  * memory); clear != 0 resets the word.  No counterpart in the reference. */
 int pado_device_status(pado_op_t op, int clear);
 /* The kernel a forward apply with these arguments would launch (nothing is
- * launched): info[0] kernel variant (1..6; the register kernel: 4 or 6, the
- * copies that feed it), [1] lines per tile, [2] stages,
- * [3] CTAs per SM, [4] segments per line, [5] coupling window, [6] threads
- * per CTA, [7] dynamic shared memory bytes.  No counterpart in the reference. */
+ * launched): info[0] kernel variant (1..6; the register kernel has none of
+ * its own and reports 4 for the fields that 4 can run on, 6 for others), [1]
+ * lines per tile, [2] stages, [3] CTAs per SM, [4] segments per line, [5]
+ * coupling window, [6] threads per CTA, [7] dynamic shared memory bytes.  No
+ * counterpart in the reference. */
 int pado_launch_plan(pado_op_t op, int kind, int axis, const double *f, double *df, long na, long nb, int bc1,
                      int bcn, int *info);
+/* 1 when a forward apply with these arguments would launch the register
+ * kernel, 0 when another one or nothing, or an error code (negative, or 324).
+ * No counterpart in the reference. */
+int pado_launch_is_register(pado_op_t op, int kind, int axis, const double *f, double *df, long na, long nb, int bc1,
+                            int bcn);
 
 /* ---- batched execution (many fields, one persistent launch) ------------ */
 

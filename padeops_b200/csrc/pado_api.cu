@@ -1161,6 +1161,24 @@ int pado_set_kernel_variant(pado_op_t op, int variant)
     return PADO_OK;
 }
 
+// The register kernel's launch of a stored forward apply; false when another kernel runs it.
+static bool plan_reg_forward(const pado_op_s *op, int kind, int axis, const double *f, double *df, long na, long nb,
+                             int bc1, int bcn, RegLaunch *r)
+{
+    const RegOp *ro = reg_op(op, kind, axis, bc1, bcn, false, SAME_BC, SAME_BC);
+    return ro && plan_reg_op(op, *ro, kind, axis, f, df, na, nb, false, OUT_STORE, 1.0, r);
+}
+
+int pado_launch_is_register(pado_op_t op, int kind, int axis, const double *f, double *df, long na, long nb, int bc1,
+                            int bcn)
+{
+    bool trivial = true;
+    const int rc = check_request(op, kind, axis, f, df, na, nb, bc1, bcn, &trivial);
+    if (rc != PADO_OK || trivial) return rc;
+    RegLaunch r;
+    return plan_reg_forward(op, kind, axis, f, df, na, nb, bc1, bcn, &r) ? 1 : 0;
+}
+
 int pado_launch_plan(pado_op_t op, int kind, int axis, const double *f, double *df, long na, long nb, int bc1,
                      int bcn, int *info)
 {
@@ -1170,20 +1188,18 @@ int pado_launch_plan(pado_op_t op, int kind, int axis, const double *f, double *
     bool trivial = true;
     int rc = prepare_launch(op, kind, axis, f, df, na, nb, bc1, bcn, false, op ? op->lines : 0, false, &kp, &trivial);
     if (rc != PADO_OK || trivial) return rc;
-    if (const RegOp *ro = reg_op(op, kind, axis, bc1, bcn, false, SAME_BC, SAME_BC)) {
-        RegLaunch r;
-        if (plan_reg_op(op, *ro, kind, axis, f, df, na, nb, false, OUT_STORE, 1.0, &r)) {
-            const bool copies = r.mode == REG_PACK || r.mode == REG_ODD || r.kp.async_copy;
-            info[0] = copies ? 6 : 4;
-            info[1] = r.lines;
-            info[2] = r.kp.stages;
-            info[3] = r.ctas;
-            info[4] = r.kp.S;
-            info[5] = r.kp.W;
-            info[6] = r.threads;
-            info[7] = (int)r.smem;
-            return PADO_OK;
-        }
+    RegLaunch r;
+    if (plan_reg_forward(op, kind, axis, f, df, na, nb, bc1, bcn, &r)) {
+        const bool copies = r.mode == REG_PACK || r.mode == REG_ODD || r.kp.async_copy;
+        info[0] = copies ? 6 : 4;
+        info[1] = r.lines;
+        info[2] = r.kp.stages;
+        info[3] = r.ctas;
+        info[4] = r.kp.S;
+        info[5] = r.kp.W;
+        info[6] = r.threads;
+        info[7] = (int)r.smem;
+        return PADO_OK;
     }
     info[4] = kp.S;
     info[5] = kp.W;

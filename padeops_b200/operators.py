@@ -109,12 +109,13 @@ class _Scheme:
 
     def launch_plan(self, kind: int, axis: int, f: torch.Tensor, df: torch.Tensor, na: int, nb: int,
                     bc1: int = 0, bcn: int = 0) -> dict:
-        """The kernel and tiling a forward apply with these arguments would use."""
+        """The kernel and tiling a forward apply with these arguments would use ("register": the register
+        kernel, whose "variant" is 4 for the fields that 4 can run on, 6 for others)."""
         info = (ctypes.c_int * 8)()
-        check(L.lib().pado_launch_plan(self.handle, kind, axis, ctypes.c_void_p(f.data_ptr()),
-                                       ctypes.c_void_p(df.data_ptr()), na, nb, bc1, bcn, info), "launch_plan")
+        args = (self.handle, kind, axis, f.data_ptr(), df.data_ptr(), na, nb, bc1, bcn)
+        check(L.lib().pado_launch_plan(*args, info), "launch_plan")
         keys = ("variant", "lines", "stages", "ctas_per_sm", "segments", "window", "threads", "smem")
-        return dict(zip(keys, list(info)))
+        return dict(zip(keys, list(info)), register=L.lib().pado_launch_is_register(*args) == 1)
 
     def set_stream_tiling(self, lines: int = 0, stages: int = 0) -> None:
         """Lines per tile and shared-memory stages of the streaming kernel (0 = automatic)."""

@@ -1,8 +1,10 @@
 """GPU: the register kernel (the automatic choice for lines of 24 points and
-more) on fields of more tiles than resident CTAs, at line lengths on the edges
-of its cuts -- no shared rows, the most, one segment -- and partial tiles and
-chunks, through both copy paths, against the oracle (1e-12 of max |oracle|);
-and the same field through the streaming kernel, the path it replaced."""
+more) against the oracle (1e-12 of max |oracle|): at line lengths on the edges
+of its cuts -- no shared rows, the most, one segment -- with partial tiles and
+chunks, and the same field through the streaming kernel, the path it replaced;
+every tile layout and copy form on fields of more tiles than resident CTAs,
+stored, scaled and accumulated.  Every case asserts that the kernel is the one
+that would run."""
 import numpy as np
 import pytest
 
@@ -37,7 +39,7 @@ def test_register_kernel(scheme, kind, n):
                 na, nb = na_nb(shape, axis)
                 out = torch.full_like(ft, float("nan"))
                 plan = op.launch_plan(kind, axis, ft, out, na, nb, *bc)
-                assert plan["variant"] == (6 if odd else 4)
+                assert plan["variant"] == (6 if odd else 4) and plan["register"]
                 op.apply(kind, axis, ft, out, na, nb, *bc)
                 torch.cuda.synchronize()
                 assert op.device_status() == 0
@@ -45,6 +47,7 @@ def test_register_kernel(scheme, kind, n):
                 assert rel_err(out.cpu().numpy(), ref) <= TOL, (periodic, axis, odd)
                 general = torch.full_like(ft, float("nan"))
                 op.set_variant(plan["variant"])
+                assert not op.launch_plan(kind, axis, ft, general, na, nb, *bc)["register"]
                 op.apply(kind, axis, ft, general, na, nb, *bc)
                 op.set_variant(0)
                 assert rel_err(out.cpu().numpy(), general.cpu().numpy()) <= TOL, (periodic, axis, odd)
@@ -63,11 +66,70 @@ def test_register_kernel_long_lines(scheme, kind, n):
             ft = torch.from_numpy(f).cuda()
             na, nb = na_nb(shape, axis)
             out = torch.full_like(ft, float("nan"))
+            assert op.launch_plan(kind, axis, ft, out, na, nb)["register"]
             op.apply(kind, axis, ft, out, na, nb)
             torch.cuda.synchronize()
             assert op.device_status() == 0
             ref = _oracle_apply(scheme, kind, axis, f, 0.3, periodic, 0, 0)
             assert rel_err(out.cpu().numpy(), ref) <= TOL, (periodic, axis)
+
+
+def _at(torch, a, offset):
+    """A device copy of the array that starts `offset` elements past a 16-byte boundary."""
+    t = torch.empty(a.size + offset, dtype=torch.float64, device="cuda")[offset:].view(a.shape)
+    t.copy_(torch.from_numpy(a))
+    return t
+
+
+# axis, rows, cross extent, elements past a 16-byte boundary, stages
+TILES = [
+    (1, 64, 83, 0, 2),     # swizzled, two buffers
+    (1, 100, 83, 0, 2),    # the same with a partial chunk
+    (1, 1800, 9, 0, 1),    # swizzled, one buffer
+    (1, 127, 83, 0, 2),    # one span each way, two buffers
+    (1, 511, 21, 0, 2),
+    (1, 96, 83, 1, 1),     # per-element copies
+    (2, 100, 70, 0, 1),    # boxes of rows
+    (3, 512, 70, 0, 1),    # more rows than a box holds
+    (2, 100, 71, 0, 1),    # rows of either parity apart: every plane starts on the same one
+    (2, 101, 71, 0, 1),    # ... on another one each
+    (3, 90, 71, 0, 1),
+    (2, 100, 70, 1, 1),    # per-element copies
+    (3, 129, 71, 1, 1),
+]
+
+
+@pytest.mark.parametrize("scheme,kind", OPS)
+@pytest.mark.parametrize("axis,n,cross,offset,stages", TILES)
+def test_register_kernel_many_tiles(scheme, kind, axis, n, cross, offset, stages):
+    import torch
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    rng = np.random.default_rng(n + 7 * axis + 3 * scheme + kind)
+    for periodic in (True, False):
+        op = _make(scheme, n, 0.3, periodic)
+        bc = (0, 0) if periodic or scheme == oracle.CD06 else (1, -1)
+        planes = 9
+        while True:  # as many planes as give every CTA two tiles and more
+            shape = {1: (planes, cross, n), 2: (planes, n, cross), 3: (n, planes, cross)}[axis]
+            na, nb = na_nb(shape, axis)
+            ft = _at(torch, np.zeros(shape), offset)
+            plan = op.launch_plan(kind, axis, ft, _at(torch, np.zeros(shape), offset), na, nb, *bc)
+            assert plan["register"] and plan["stages"] == stages, plan
+            L = plan["lines"]
+            tiles = -(-na // L) * nb if axis == 2 else -(-na * nb // L)
+            if tiles > 2 * plan["ctas_per_sm"] * sms:
+                break
+            planes = 2 * planes + 1
+        f, df0 = rng.standard_normal(shape), rng.standard_normal(shape)
+        ft = _at(torch, f, offset)
+        ref = _oracle_apply(scheme, kind, axis, f, 0.3, periodic, *bc)
+        for alpha, beta in ((1.0, 0.0), (-0.75, 0.0), (-0.75, 1.0)):
+            out = _at(torch, df0 if beta else np.full(shape, np.nan), offset)
+            op.apply(kind, axis, ft, out, na, nb, *bc, alpha=alpha, beta=beta)
+            expect = alpha * ref + beta * df0
+            assert rel_err(out.cpu().numpy(), expect) <= TOL, (periodic, alpha, beta)
+        assert op.device_status() == 0
 
 
 @pytest.mark.parametrize("scheme,kind", OPS)
@@ -88,7 +150,7 @@ def test_register_kernel_odd_lines_one_buffer(scheme, kind, n, n2, n3):
         out = torch.empty_like(ft)
         plan = op.launch_plan(kind, 1, ft, out, n2, n3)
         tiles = -(-n2 * n3 // plan["lines"])
-        assert plan["stages"] == 1 and tiles > plan["ctas_per_sm"] * sms, plan
+        assert plan["register"] and plan["stages"] == 1 and tiles > plan["ctas_per_sm"] * sms, plan
         assert n2 * n3 % plan["lines"] == plan["lines"] - 1
         ref = _oracle_apply(scheme, kind, 1, f, 0.3, periodic, 0, 0)
         for alpha, beta in ((1.0, 0.0), (-0.75, 1.0)):

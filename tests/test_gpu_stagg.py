@@ -35,6 +35,7 @@ def _gpu(torch, st, name, f):
     out = torch.full((nout,) + f.shape[1:], float("nan"), dtype=ft.dtype, device="cuda")
     getattr(st, name)(ft, out, f.shape[2], f.shape[1])
     torch.cuda.synchronize()
+    assert st.device_status() == 0
     return out.cpu().numpy()
 
 
@@ -135,3 +136,22 @@ def test_stagg_errors(torch_cuda):
         st.ddz_E2C(f, f[: 8 * 4], 2, 2)  # overlapping input and output
     with pytest.raises(ValueError):
         st.ddz_E2C(f.cpu(), torch.empty(8 * 4, dtype=torch.float64), 2, 2)  # no CPU path
+
+
+@pytest.mark.parametrize("n1,n2", [(420, 211), (421, 211)])
+def test_stagg_many_tiles(torch_cuda, n1, n2):
+    """More tiles of 32 lines than 148 SMs hold CTAs, lines an even and an odd number of elements apart."""
+    import padeops_b200 as pb
+
+    torch, n = torch_cuda, 48
+    rng = np.random.default_rng(n1)
+    for setup in (dict(periodic=True), dict(periodic=False, top_even=True, bot_even=False, top_sided=False, bot_sided=True)):
+        S, st = Stagg(n, 0.1, **setup), pb.cd06stagg()
+        closures = [setup[k] for k in ("top_even", "bot_even", "top_sided", "bot_sided")] if not setup["periodic"] else []
+        assert st.init(n, 0.1, *closures) == 0
+        for name in OPS:
+            if setup["periodic"] and name in ("ddz_C2C", "ddz_E2E"):
+                continue
+            f = rng.standard_normal((st.sizes(name)[0], n2, n1))
+            assert rel_err(_gpu(torch, st, name, f), _oracle(S, name, f)) <= TOL, (setup, name)
+        st.destroy()
