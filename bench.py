@@ -490,7 +490,7 @@ def run_gpu(args) -> None:
             per_operator()
         torch.cuda.synchronize()
         el_op = (time.perf_counter() - t1) / e2e_steps
-        per_op = {"value": round(9 * N ** 3 / el_op / 1e9 * world, 3), "unit": "Gpts/s",
+        host_calls = {"value": round(9 * N ** 3 / el_op / 1e9 * world, 3), "unit": "Gpts/s",
                   "h2d_bytes_per_step": 9 * field_bytes, "d2h_bytes_per_step": 9 * field_bytes,
                   "path": "pado_apply_host per operator (pinned host buffers)"}
         if terms_path:
@@ -506,10 +506,10 @@ def run_gpu(args) -> None:
             e2e = {"value": 9 * N ** 3 / el / 1e9 * world, "unit": "Gpts/s",
                    "h2d_bytes_per_step": field_bytes, "d2h_bytes_per_step": 9 * field_bytes,
                    "path": "pado_apply_host_terms: one upload of f, nine results downloaded (pinned host buffers)",
-                   "per_operator_host_calls": per_op}
+                   "per_operator_host_calls": host_calls}
             del houts
         else:
-            e2e = dict(per_op)
+            e2e = dict(host_calls)
 
     cpu = None
     if rank == 0 and world == 1 and not args.no_cpu:
