@@ -59,8 +59,8 @@ def measured_peaks() -> tuple[float, str]:
 
 
 def profiled_traffic() -> float | None:
-    """DRAM bytes per 512^3 launch of the register kernel from the committed ncu
-    summary (profiles/register_kernel_512cube.md, line 'traffic_bytes_per_launch: X')."""
+    """DRAM bytes of one 512^3 launch of the register kernel, cd10 d1 along z, from the committed
+    ncu summary (profiles/register_kernel_512cube.md, line 'traffic_bytes_per_launch: X')."""
     p = os.path.join(ROOT, "profiles", "register_kernel_512cube.md")
     try:
         with open(p) as fh:
@@ -491,8 +491,8 @@ def run_gpu(args) -> None:
         torch.cuda.synchronize()
         el_op = (time.perf_counter() - t1) / e2e_steps
         host_calls = {"value": round(9 * N ** 3 / el_op / 1e9 * world, 3), "unit": "Gpts/s",
-                  "h2d_bytes_per_step": 9 * field_bytes, "d2h_bytes_per_step": 9 * field_bytes,
-                  "path": "pado_apply_host per operator (pinned host buffers)"}
+                      "h2d_bytes_per_step": 9 * field_bytes, "d2h_bytes_per_step": 9 * field_bytes,
+                      "path": "pado_apply_host per operator (pinned host buffers)"}
         if terms_path:
             houts = [hdf] + [torch.empty_like(hf).pin_memory() for _ in plan[1:]]
             terms = [(op, kind, axis, 0, 0, 1.0, 0.0, i) for i, (op, kind, axis) in enumerate(plan)]
@@ -526,7 +526,7 @@ def run_gpu(args) -> None:
                 "vs_baseline": None, "dtype": "f64", "data": "synthetic",
                 "config": dict(CONFIG, per_operator_gbs=per_op),
                 "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
-                             "frac": round(achieved / peak, 4), "traffic": profiled_traffic(),
+                             "frac": round(achieved / peak, 4), "traffic": profiled_traffic(), "traffic_of": "cd10 d1 along z, one launch (ncu)",
                              "kernel": "pado::reg_kernel (the 9 launches of a step, averaged)",
                              "peak_source": peak_kind},
                 "cpu_baseline": cpu, "e2e": e2e, "clocks": clk.summary(), "gpu_launches": launches,

@@ -52,7 +52,8 @@ class Batch:
 
     def set_graph_branches(self, branches: int) -> int:
         """What run_graph captures: 0 = the persistent launch, k > 0 = one
-        streaming-kernel launch per item on k concurrent graph branches."""
+        launch per item (the kernel an apply would take) on k concurrent graph
+        branches (96 uneven fields: 1.4 ms against the persistent launch's 3.6)."""
         return L.lib().pado_batch_set_graph_branches(self._h, branches)
 
     def set_config(self, lines: int = 0, ctas_per_sm: int = 0) -> int:

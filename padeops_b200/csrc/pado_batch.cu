@@ -25,8 +25,8 @@ struct pado_batch_s {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     cudaStream_t capture_stream = nullptr;
-    // graph contents: 0 = the persistent launch; k > 0 = one streaming-kernel
-    // launch per item, the items dealt round-robin to k concurrent branches
+    // graph contents: 0 = the persistent launch; k > 0 = one launch per item,
+    // the items dealt largest first to k concurrent branches
     int branches = 0;
     std::vector<cudaStream_t> branch_streams;
     std::vector<cudaEvent_t> branch_events;  // [0]: fork, [1 + k]: branch k done

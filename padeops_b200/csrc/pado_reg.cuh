@@ -37,15 +37,15 @@
 // 5e-6), so the near-singular A (condition number near 2000) amplifies the
 // rounding of d and not that of f; f is added when d is complete.
 //
-// What bounds it: HBM, at 90-95% of the measured copy rate (6448 GB/s) for the
-// derivatives and 81-95% for cf90.  Per point the kernel issues the stencil (5
+// What bounds it: HBM, at 82-96% of the measured copy rate (6448 GB/s) for the
+// derivatives of 512-row lines and 81-87% for cf90.  Per point the kernel issues the stencil (5
 // to 10 FP64), 4 recurrence and 4 correction FMAs, 1 + 2 H / M shared loads (H
 // the stencil's half width) and one store -- 31 (cd10 d1) to 56 (bounded cf90)
 // instructions in all -- against 67 to 90 of the streaming kernel, which keeps
 // the line in shared memory and passes over it four times.  B200, 512^3, x + y
-// + z, streaming kernel -> this kernel: cd10 d1 1929 -> 1070 us, cd10 d2 1985
-// -> 1065 us, cf90 2319 -> 1111 us; 1024x512x256 with walls in z: cd06 1664 ->
-// 1096 us, cd10 d1 1999 -> 1079 us.
+// + z, streaming kernel -> this kernel: cd10 d1 1929 -> 1057 us, cd10 d2 1985
+// -> 1106 us, cf90 2319 -> 1145 us; 1024x512x256 with walls in z: cd06 1664 ->
+// 1107 us, cd10 d1 1999 -> 1099 us.
 #pragma once
 
 #include <cuda.h>
@@ -62,8 +62,9 @@ constexpr int REG_MAXM = 32;      // longest segment
 constexpr int REG_MAXS = 64;      // most segments per line
 constexpr int REG_EDGE = 4;       // closure rows solved as a block at each end
 // Most rows two neighbouring segments of M share: with 8 of 32 every line of
-// 104 points or more cuts into 32s (cd06 of 99 rows 5100 -> 5660 GB/s along y,
-// cd10 d2 of 64 rows with walls 4820 -> 5780; with 4 such lines took 16s).
+// 104 rows or more between its closure blocks (112 points with walls) cuts into
+// 32s, and some shorter ones (walls, along y: cd06 of 99 points 5100 -> 5660
+// GB/s, cd10 d2 of 64 points 4820 -> 5780; with 4 such lines took 16s).
 PADO_HD constexpr int reg_overlap(int M) { return M >= 32 ? 8 : 4; }
 constexpr int REG_SEGTAB = 12;    // doubles per segment of the edge tables
 // Closure rows of the staggered scheme, as its right-hand sides group them:

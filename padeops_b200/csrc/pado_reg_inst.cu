@@ -6,7 +6,7 @@
 #include "pado_internal.h"
 
 #if !defined(PADO_RK) || !defined(PADO_RM)
-#error "compile with -DPADO_RK=<stencil 0..3> -DPADO_RM=<rows per segment>"
+#error "compile with -DPADO_RK=<stencil 0..7> -DPADO_RM=<rows per segment>"
 #endif
 #define PADO_CAT4(a, b, c, d) a##b##c##d
 #define PADO_CAT(a, b, c, d) PADO_CAT4(a, b, c, d)

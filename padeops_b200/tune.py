@@ -130,9 +130,9 @@ def _time(fn, reps: int) -> float:
 
 def tune_batch(batch, reps: int = 5, verbose: bool = False, branches=(0, 2, 4, 8)) -> tuple[int, int, int, float]:
     """Autotune a batch: the persistent kernel's (lines per tile, CTAs per SM),
-    then what its CUDA graph holds -- the persistent launch (0) or one
-    streaming-kernel launch per item on k concurrent branches -- by timing the
-    graph replay.  Returns (lines, ctas_per_sm, branches, ms); 0 means
+    then what its CUDA graph holds -- the persistent launch (0) or one launch
+    per item, of the kernel an apply would take, on k concurrent branches -- by
+    timing the graph replay.  Returns (lines, ctas_per_sm, branches, ms); 0 means
     automatic / no cap / the persistent launch."""
     best = None
     for lines in (0, 8, 16, 32):
