@@ -425,11 +425,36 @@ bool plan_stream(const pado_op_s *op, const DevTables &dt, const KParams &kp0, i
     return true;
 }
 
-bool plan_reg_op(const pado_op_s *op, const RegOp &ro, int kind, int axis, const double *f, double *df, long long na,
-                 long long nb, bool adj, int out_mode, double out_alpha, RegLaunch *out)
+// The register kernel's constants for a request, or null when another kernel
+// runs it: an explicit kernel or tiling, a short or uncuttable line, the
+// adjoint of a bounded line.
+const RegOp *reg_op(const pado_op_s *op, int kind, int axis, int bc1, int bcn, bool adj, int solve_bc1, int solve_bcn)
 {
+    if (op->variant != 0 || op->stream_lines || op->stream_stages || op->tiled || (adj && !op->periodic)) return nullptr;
+    const bool bounded_bc = !op->periodic && op->scheme != CD06;
+    const int b1 = bounded_bc ? bc1 : 0, bn = bounded_bc ? bcn : 0;
+    const int s1 = bounded_bc && solve_bc1 != SAME_BC ? solve_bc1 : b1, sn = bounded_bc && solve_bcn != SAME_BC ? solve_bcn : bn;
+    const auto it = op->reg.find(RegKey(kind, b1, bn, s1, sn, reg_even_starts(axis, op->n) ? 1 : 0));
+    return it == op->reg.end() ? nullptr : it->second.get();
+}
+
+// The register kernel's launch for a request; false when another kernel runs it.
+bool plan_register(const pado_op_s *op, int kind, int axis, const double *f, double *df, long long na, long long nb,
+                   int bc1, int bcn, bool adj, int solve_bc1, int solve_bcn, int out_mode, double out_alpha,
+                   RegLaunch *out)
+{
+    // y lines of a field one point wide lie one after another, as x lines do;
+    // as strided ones each would be a tile of its own (adjoint of cf90 on 25
+    // rows, 203594 such lines: 268 us, 89 in the line kernel)
+    if (axis == 2 && na == 1) {
+        axis = 1;
+        na = nb;
+        nb = 1;
+    }
+    const RegOp *ro = reg_op(op, kind, axis, bc1, bcn, adj, solve_bc1, solve_bcn);
+    if (!ro) return false;
     RegParams &kp = out->kp;
-    kp = ro.kp;
+    kp = ro->kp;
     kp.in = f;
     kp.out = df;
     kp.nlines = na * nb;
@@ -446,20 +471,7 @@ bool plan_reg_op(const pado_op_s *op, const RegOp &ro, int kind, int axis, const
     const int rk = rhs_kind_of(op->scheme, kind);
     if (adj && (rk == RHS_CD06_D1 || rk == RHS_CD10_D1))
         for (double &t : kp.taps) t = -t;  // a cyclic first derivative is antisymmetric, the others symmetric
-    return plan_reg(rk, op->periodic != 0, ro.cut, na, nb, out);
-}
-
-// The register kernel's constants for a request, or null when another kernel
-// runs it: an explicit kernel or tiling, a short or uncuttable line, the
-// adjoint of a bounded line.
-const RegOp *reg_op(const pado_op_s *op, int kind, int axis, int bc1, int bcn, bool adj, int solve_bc1, int solve_bcn)
-{
-    if (op->variant != 0 || op->stream_lines || op->stream_stages || op->tiled || (adj && !op->periodic)) return nullptr;
-    const bool bounded_bc = !op->periodic && op->scheme != CD06;
-    const int b1 = bounded_bc ? bc1 : 0, bn = bounded_bc ? bcn : 0;
-    const int s1 = bounded_bc && solve_bc1 != SAME_BC ? solve_bc1 : b1, sn = bounded_bc && solve_bcn != SAME_BC ? solve_bcn : bn;
-    const auto it = op->reg.find(RegKey(kind, b1, bn, s1, sn, reg_even_starts(axis, op->n) ? 1 : 0));
-    return it == op->reg.end() ? nullptr : it->second.get();
+    return plan_reg(rk, op->periodic != 0, ro->cut, na, nb, out);
 }
 
 // SMs of the current device, asked of the runtime once per device.
@@ -773,10 +785,9 @@ int launch(pado_op_s *op, int kind, int axis, const double *f, double *df, long 
         }
         return e == cudaSuccess ? PADO_OK : cuda_fail(e);
     }
-    if (const RegOp *ro = reg_op(op, kind, axis, bc1, bcn, adjoint, solve_bc1, solve_bcn)) {
-        RegLaunch r;
-        if (plan_reg_op(op, *ro, kind, axis, f, df, na, nb, adjoint, out_mode, out_alpha, &r)) return launch_reg(r, st);
-    }
+    RegLaunch r;
+    if (plan_register(op, kind, axis, f, df, na, nb, bc1, bcn, adjoint, solve_bc1, solve_bcn, out_mode, out_alpha, &r))
+        return launch_reg(r, st);
     KParams kp;
     rc = prepare_launch(op, kind, axis, f, df, na, nb, bc1, bcn, adjoint, op->lines, false, &kp, &trivial, solve_bc1,
                         solve_bcn, out_mode, out_alpha);
@@ -1161,14 +1172,6 @@ int pado_set_kernel_variant(pado_op_t op, int variant)
     return PADO_OK;
 }
 
-// The register kernel's launch of a stored forward apply; false when another kernel runs it.
-static bool plan_reg_forward(const pado_op_s *op, int kind, int axis, const double *f, double *df, long na, long nb,
-                             int bc1, int bcn, RegLaunch *r)
-{
-    const RegOp *ro = reg_op(op, kind, axis, bc1, bcn, false, SAME_BC, SAME_BC);
-    return ro && plan_reg_op(op, *ro, kind, axis, f, df, na, nb, false, OUT_STORE, 1.0, r);
-}
-
 int pado_launch_is_register(pado_op_t op, int kind, int axis, const double *f, double *df, long na, long nb, int bc1,
                             int bcn)
 {
@@ -1176,7 +1179,7 @@ int pado_launch_is_register(pado_op_t op, int kind, int axis, const double *f, d
     const int rc = check_request(op, kind, axis, f, df, na, nb, bc1, bcn, &trivial);
     if (rc != PADO_OK || trivial) return rc;
     RegLaunch r;
-    return plan_reg_forward(op, kind, axis, f, df, na, nb, bc1, bcn, &r) ? 1 : 0;
+    return plan_register(op, kind, axis, f, df, na, nb, bc1, bcn, false, SAME_BC, SAME_BC, OUT_STORE, 1.0, &r) ? 1 : 0;
 }
 
 int pado_launch_plan(pado_op_t op, int kind, int axis, const double *f, double *df, long na, long nb, int bc1,
@@ -1189,7 +1192,7 @@ int pado_launch_plan(pado_op_t op, int kind, int axis, const double *f, double *
     int rc = prepare_launch(op, kind, axis, f, df, na, nb, bc1, bcn, false, op ? op->lines : 0, false, &kp, &trivial);
     if (rc != PADO_OK || trivial) return rc;
     RegLaunch r;
-    if (plan_reg_forward(op, kind, axis, f, df, na, nb, bc1, bcn, &r)) {
+    if (plan_register(op, kind, axis, f, df, na, nb, bc1, bcn, false, SAME_BC, SAME_BC, OUT_STORE, 1.0, &r)) {
         const bool copies = r.mode == REG_PACK || r.mode == REG_ODD || r.kp.async_copy;
         info[0] = copies ? 6 : 4;
         info[1] = r.lines;

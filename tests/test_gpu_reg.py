@@ -207,3 +207,36 @@ def test_rounding_does_not_depend_on_the_address(scheme, kind):
                 for out in outs[1:]:
                     assert torch.equal(out, outs[0]), (n, periodic, axis, cross)
             assert op.device_status() == 0
+
+
+@pytest.mark.parametrize("scheme,kind", OPS)
+@pytest.mark.parametrize("n", [25, 64, 129])
+def test_lines_across_a_field_one_point_wide(scheme, kind, n):
+    """y lines of a field of extent 1 along x follow one another in memory: they are tiled as x lines, stored,
+    accumulated and transposed, and give an x line's bits."""
+    import torch
+
+    rng = np.random.default_rng(n + scheme + kind)
+    f = rng.standard_normal((2003, n, 1))
+    ft = torch.from_numpy(f).cuda()
+    for periodic in (True, False):
+        op = _make(scheme, n, 0.3, periodic)
+        outs = [torch.full_like(ft, float("nan")) for _ in range(2)]
+        plans = [op.launch_plan(kind, axis, ft, out, na, nb)
+                 for out, axis, na, nb in zip(outs, (2, 1), (1, 2003), (2003, 1))]
+        assert plans[0]["register"] and plans[0] == plans[1]
+        op.apply(kind, 2, ft, outs[0], 1, 2003)
+        op.apply(kind, 1, ft, outs[1], 2003, 1)
+        assert torch.equal(*outs)
+        assert rel_err(outs[0].cpu().numpy(), _oracle_apply(scheme, kind, 2, f, 0.3, periodic, 0, 0)) <= TOL
+        acc = [ft.clone(), ft.clone()]
+        op.apply(kind, 2, ft, acc[0], 1, 2003, alpha=-0.5, beta=1.0)
+        op.apply(kind, 1, ft, acc[1], 2003, 1, alpha=-0.5, beta=1.0)
+        assert torch.equal(*acc)
+        adj = torch.full_like(ft, float("nan"))
+        op.apply(kind, 2, ft, adj, 1, 2003, adjoint=True)
+        g = torch.from_numpy(rng.standard_normal(f.shape)).cuda()
+        op.apply(kind, 2, g, outs[1], 1, 2003)
+        bound = 1e-12 * float(outs[1].norm() * ft.norm())
+        assert abs(float((outs[1] * ft).sum()) - float((g * adj).sum())) <= bound, periodic
+        assert op.device_status() == 0
